@@ -10,6 +10,7 @@
 // counter.  Every job's output is bit-identical to the per-scene kernels of trace.cu for
 // the same grid, camera, samples, seed and image ids: the per-pixel random streams, ray
 // construction and traversal are the same functions.
+#define HR_TRAV_WARPS 8   // blocks of up to 256 threads
 #include "traverse.cuh"
 #include "../../include/happyray.h"
 

@@ -303,7 +303,7 @@ __global__ __launch_bounds__(kTT, HR_TRACE_MIN_BLOCKS) void k_ao_primary_tl(Scen
         if (!__any_sync(kFullMask, has)) break;   // the pool is dry and no ray is in flight
         uint32_t b = 0, e = 0;
         if (active) {
-            const uint2 lr = __ldg(s.leaves + tl_leaf(q));
+            const uint2 lr = __ldg(s.leaves + q.leaf);
             b = lr.x; e = lr.y;
             if (STATS) h.cells++;
         }
@@ -404,7 +404,7 @@ __global__ __launch_bounds__(kTT, HR_TRACE_MIN_BLOCKS) void k_ao_samples_tl(Scen
         if (!__any_sync(kFullMask, has)) break;   // the pool is dry and no ray is in flight
         uint32_t b = 0, e = 0;
         if (active) {
-            const uint2 lr = __ldg(s.leaves + tl_leaf(q));
+            const uint2 lr = __ldg(s.leaves + q.leaf);
             b = lr.x; e = lr.y;
             if (STATS) h.cells++;
         }

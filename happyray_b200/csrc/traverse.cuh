@@ -113,23 +113,37 @@ constexpr int kHitClosest = 0, kHitAny = 1, kHitMixed = 2;
 __device__ __forceinline__ float shfl(float x, int src) { return __shfl_sync(kFullMask, x, src); }
 __device__ __forceinline__ uint32_t shfl(uint32_t x, int src) { return __shfl_sync(kFullMask, x, src); }
 
+#ifndef HR_TRAV_WARPS
+#define HR_TRAV_WARPS 4   // warps of the largest block that traverses
+#endif
+
 // Warp-wide test of every lane's list prims[b, e); must be called by all 32 lanes, and
 // returns true on the lanes whose any-hit query it answers.  The (lane, triangle) pairs of
 // all lanes are numbered in lane order and tested 32 per round, one pair per lane, so no
-// lane idles while another walks a longer list.  Pair j belongs to the lane whose
-// [exclusive, inclusive) prefix of list lengths holds j and is tested with that lane's
-// ray and current bound.  Closest hit: the hits of a round are applied one by one in pair
-// order, each only if its t is strictly below the lane's best so far -- the
-// first-tested-wins rule of a one-lane loop over the list.  Any hit: a lane is answered
-// when one of its pairs hits; its later pairs are skipped.  STATS counts the pairs
-// tested: all of a list for closest hit (as the sequential loop), whole rounds for any hit.
+// lane idles while another walks a longer list.  Pair j belongs to the last list that
+// starts at or before j: the round's list starts are one bit per lane (or-reduced), their
+// count up to j numbers the list, and a byte table in shared memory names its lane; the
+// pair is tested with that lane's ray and current bound.  Closest hit: the hits of a round
+// are applied by their owners in pair order, each only if its t is strictly below the
+// lane's best so far -- the first-tested-wins rule of a one-lane loop over the list.  Any
+// hit: a lane is answered when one of its pairs hits; rounds that hold only pairs of
+// answered lanes are skipped.  STATS counts the pairs tested: all of a list for closest
+// hit (as the sequential loop), whole rounds for any hit.
+//
+// The kernels are bound by instruction issue and by the latency of a round, so a round
+// spends as little as it can beside the test: finding the owner by a five-step search over
+// the lists' prefix sums and applying hits one by one for the whole warp cost c2's AO
+// 1.84 ms against 1.80, c1's camera rays 0.069 against 0.066, a uniform grid with lists of
+// thousands 2.90 against 2.59; rays read from shared memory instead of by shuffles 1.84
+// (and 1.70 against 1.53 in the job kernel, whose L1 the copies crowd).
 template <int HM, bool STATS>
 __device__ __forceinline__ bool test_lists(const Scene& s, f3 o, f3 d, uint32_t b, uint32_t e, bool any, Hit& h) {
+    __shared__ uint8_t s_lane[HR_TRAV_WARPS][32];
     const uint32_t lane = threadIdx.x & 31u;
     const uint32_t n = e - b;
-    if (__ballot_sync(kFullMask, n != 0u) == 0u) return false;   // most leaves a ray crosses are empty
-    // lanes whose query is an any-hit query
-    const uint32_t anym = HM == kHitAny ? kFullMask : (HM == kHitClosest ? 0u : __ballot_sync(kFullMask, any));
+    const uint32_t ne = __ballot_sync(kFullMask, n != 0u);
+    if (ne == 0u) return false;   // most leaves a ray crosses are empty
+    uint8_t* const lane_of = s_lane[threadIdx.x >> 5];   // lane of the k-th non-empty list
     uint32_t incl = n;
 #pragma unroll
     for (int off = 1; off < 32; off <<= 1) {
@@ -137,80 +151,90 @@ __device__ __forceinline__ bool test_lists(const Scene& s, f3 o, f3 d, uint32_t 
         if (lane >= (uint32_t)off) incl += x;
     }
     const uint32_t total = __shfl_sync(kFullMask, incl, 31);
+    const uint32_t excl = incl - n;
+    if (n != 0u) lane_of[__popc(ne & ((1u << lane) - 1u))] = (uint8_t)lane;
+    __syncwarp();
     // prims index of pair j of this lane: rel + j, summed in 32 bits (rel wraps when b is
     // below the lane's exclusive prefix; the sum does not)
-    const uint32_t rel = b - (incl - n);
-    uint32_t best = 0xffffffffu;           // pair number of this lane's best hit of this call
-    uint32_t answered = 0u;                // any-hit lanes with a hit
-    for (uint32_t base = 0; base < total; base += 32u) {
+    const uint32_t rel = b - excl;
+    const bool my_any = HM == kHitAny || (HM == kHitMixed && any);
+    bool answered = false;            // any-hit lanes with a hit
+    uint32_t started = 0xffffffffu;   // lists started before the round, minus one
+    for (uint32_t base = 0; base < total;) {
         const uint32_t j = base + lane;
-        uint32_t own = 0;                  // number of lanes whose inclusive prefix is <= j
-#pragma unroll
-        for (uint32_t step = 16; step > 0; step >>= 1) {
-            if (__shfl_sync(kFullMask, incl, own + step - 1u) <= j) own += step;
-        }
+        const uint32_t rs = excl - base;
+        const uint32_t heads = __reduce_or_sync(kFullMask, (n != 0u && rs < 32u) ? 1u << rs : 0u);
+        const int own = lane_of[started + __popc(heads & (0xffffffffu >> (31u - lane)))];
         const f3 so = mk(shfl(o.x, own), shfl(o.y, own), shfl(o.z, own));
         const f3 sd = mk(shfl(d.x, own), shfl(d.y, own), shfl(d.z, own));
         const float bt = shfl(h.t, own);
         const uint32_t srel = shfl(rel, own);
-        const bool own_any = (anym >> own) & 1u;
-        const bool live = j < total && !(own_any && ((answered >> own) & 1u));
         float t = 0.0f, u = 0.0f, v = 0.0f;
+        uint32_t tri = 0;
         bool hit = false;
-        if (live) hit = mt_test(s, __ldg(s.prims + (srel + j)), so, sd, bt, &t, &u, &v);
-        if (STATS && !((anym & answered) >> lane & 1u)) {   // this lane's pairs tested in the round
-            const uint32_t lo = max(incl - n, base), hi = min(incl, base + 32u);
+        if (j < total) {
+            tri = __ldg(s.prims + (srel + j));
+            hit = mt_test(s, tri, so, sd, bt, &t, &u, &v);
+        }
+        if (STATS && !answered) {   // this lane's pairs tested in the round
+            const uint32_t lo = max(excl, base), hi = min(incl, base + 32u);
             if (hi > lo) h.tests += hi - lo;
         }
-        if (HM != kHitClosest) answered |= __reduce_or_sync(kFullMask, (hit && own_any) ? 1u << own : 0u);
-        if (HM != kHitAny) {
-            uint32_t hm = __ballot_sync(kFullMask, hit && !own_any);
-            while (hm) {
-                const int src = __ffs(hm) - 1;
-                hm &= hm - 1u;
-                const uint32_t ow = shfl(own, src), hj = shfl(j, src);
-                const float ht = shfl(t, src), hu = shfl(u, src), hv = shfl(v, src);
-                if (lane == ow && ht < h.t) {
-                    h.t = ht; h.u = hu; h.v = hv; h.hit = true;
-                    best = hj;
+        const uint32_t hm = __ballot_sync(kFullMask, hit);
+        uint32_t next = base + 32u;
+        if (hm) {
+            // the round's pairs of this lane: bits [lo, hi)
+            const uint32_t lo = excl > base ? min(rs, 32u) : 0u, hi = incl > base ? min(incl - base, 32u) : 0u;
+            uint32_t m = lo < hi ? hm & ((0xffffffffu >> (32u - (hi - lo))) << lo) : 0u;
+            if (my_any) {
+                answered = answered || m != 0u;
+                m = 0u;
+            }
+            if (HM != kHitAny) {
+                while (__any_sync(kFullMask, m != 0u)) {
+                    const int src = m ? __ffs(m) - 1 : 0;
+                    const float ht = shfl(t, src), hu = shfl(u, src), hv = shfl(v, src);
+                    const uint32_t htri = shfl(tri, src);
+                    if (m != 0u && ht < h.t) {
+                        h.t = ht; h.u = hu; h.v = hv; h.hit = true; h.tri = htri;
+                    }
+                    m &= m - 1u;
                 }
             }
+            if (HM != kHitClosest && next < total) {   // the first round with a pair still to test
+                const bool left = n != 0u && !answered && incl > next;
+                next = __reduce_min_sync(kFullMask, left ? max(excl, next) : 0xffffffffu) & ~31u;
+                if (next >= total) break;
+            }
         }
+        if (next == base + 32u) started += __popc(heads);
+        else started = (uint32_t)__popc(__ballot_sync(kFullMask, n != 0u && excl < next)) - 1u;
+        base = next;
     }
-    bool done = false;
-    if (HM != kHitClosest) {
-        done = (answered >> lane) & 1u;
-        if (done) h.hit = true;
-    }
-    if (HM != kHitAny && best != 0xffffffffu) h.tri = __ldg(s.prims + (rel + best));
-    return done;
+    __syncwarp();   // the next call rewrites the table
+    if (HM != kHitClosest && answered) h.hit = true;
+    return answered;
 }
 
 __device__ __forceinline__ int min_dim(float a, float b, float c) { return a < b ? (a < c ? 0 : 2) : (b < c ? 1 : 2); }
 
-// One DDA step along the axis of the smallest tmax.  The state arrays are only indexed
-// with constants (one branch per axis, as TLGridTraverser.h:226-290 writes it out), so
-// they stay in registers.  Returns tmax of the axis before the step in *t_before and
-// whether the new cell index is inside [0, res).
-__device__ __forceinline__ bool dda_step(float* tmax, int32_t* cell, const float* rcp, const float* cs,
-                                         const int32_t* res, float* t_before) {
-    const int k = min_dim(tmax[0], tmax[1], tmax[2]);
-    if (k == 0) {
-        *t_before = tmax[0];
-        cell[0] += rcp[0] > 0.0f ? 1 : -1;
-        tmax[0] += cs[0] * fabsf(rcp[0]);
-        return cell[0] < res[0] && cell[0] > -1;
-    } else if (k == 1) {
-        *t_before = tmax[1];
-        cell[1] += rcp[1] > 0.0f ? 1 : -1;
-        tmax[1] += cs[1] * fabsf(rcp[1]);
-        return cell[1] < res[1] && cell[1] > -1;
-    } else {
-        *t_before = tmax[2];
-        cell[2] += rcp[2] > 0.0f ? 1 : -1;
-        tmax[2] += cs[2] * fabsf(rcp[2]);
-        return cell[2] < res[2] && cell[2] > -1;
-    }
+// One DDA step along the axis of the smallest t (min_dim).  `pos` is a linear index that
+// moves by the axis' signed stride st, `left` the steps that stay inside the grid per axis
+// (-1 once the step left it) and dt the axis' constant t increment, so a step is a handful
+// of predicated adds with no divergence between the axes.  (Against recomputing the cell
+// index, increment and bounds from 3-D coordinates in one branch per axis: c3 path tracing
+// 2.07 -> 1.88 ms, c2 AO 1.93 -> 1.84, shadow rays of a 500k scene 1.86 -> 1.77.)  Returns
+// whether the new cell is inside and t of the axis before the step in *t_before.
+__device__ __forceinline__ bool dda_step(float* t, const float* dt, uint32_t& pos, const uint32_t* st, int32_t* left,
+                                         float* t_before) {
+    const float a = t[0], b = t[1], c = t[2];
+    const bool ab = a < b;
+    const bool p0 = ab && a < c, p1 = !ab && b < c;
+    *t_before = p0 ? a : (p1 ? b : c);
+    if (p0) { t[0] = a + dt[0]; pos += st[0]; left[0] -= 1; }
+    if (p1) { t[1] = b + dt[1]; pos += st[1]; left[1] -= 1; }
+    if (!(p0 || p1)) { t[2] = c + dt[2]; pos += st[2]; left[2] -= 1; }
+    return (left[0] | left[1] | left[2]) >= 0;
 }
 
 __device__ __forceinline__ bool clip(const G& g, f3 o, const float* rcp, float* t0, float* t1) {
@@ -236,10 +260,12 @@ __device__ __forceinline__ bool clip(const G& g, f3 o, const float* rcp, float* 
 #endif
 template <int HM, bool STATS>
 __device__ void trace_ug(const Scene& s, const G& g, f3 o, f3 d, bool any, Hit& h, bool active) {
-    float rcp[3] = {0.0f, 0.0f, 0.0f}, tmax[3] = {0.0f, 0.0f, 0.0f};
-    int32_t cell[3] = {0, 0, 0};
+    float tmax[3] = {0.0f, 0.0f, 0.0f}, dt[3] = {0.0f, 0.0f, 0.0f};
+    int32_t left[3] = {0, 0, 0};
+    uint32_t st[3] = {0u, 0u, 0u};
+    uint32_t c = 0;   // current cell
     if (active) {
-        rcp[0] = 1.0f / d.x; rcp[1] = 1.0f / d.y; rcp[2] = 1.0f / d.z;
+        const float rcp[3] = {1.0f / d.x, 1.0f / d.y, 1.0f / d.z};
         float t0, t1;
         active = clip(g, o, rcp, &t0, &t1);
         if (active) {
@@ -248,27 +274,31 @@ __device__ void trace_ug(const Scene& s, const G& g, f3 o, f3 d, bool any, Hit& 
                 const float te = t0 + kEps;
                 ep = mk(o.x + te * d.x, o.y + te * d.y, o.z + te * d.z);
             }
+            int32_t cell[3];
+            const uint32_t stride[3] = {1u, (uint32_t)g.res[0], (uint32_t)g.res[0] * (uint32_t)g.res[1]};
 #pragma unroll
             for (int k = 0; k < 3; ++k) {
                 float cf = floorf((comp(ep, k) - g.bmin[k]) * g.rcp[k]);
                 cf = hmin((float)g.res[k] - 1.0f, hmax(cf, 0.0f));
-                const float stp = rcp[k] > 0.0f ? 1.0f : 0.0f;
+                const bool fwd = rcp[k] > 0.0f;
+                const float stp = fwd ? 1.0f : 0.0f;
                 tmax[k] = ((cf + stp) * g.cs[k] + g.bmin[k] - comp(o, k)) * rcp[k];
+                dt[k] = g.cs[k] * fabsf(rcp[k]);
                 cell[k] = f2i(cf);
+                left[k] = fwd ? g.res[k] - 1 - cell[k] : cell[k];
+                st[k] = fwd ? stride[k] : 0u - stride[k];
             }
             active = cell[0] < g.res[0] && cell[0] > -1 && cell[1] < g.res[1] && cell[1] > -1 &&
                      cell[2] < g.res[2] && cell[2] > -1;
+            c = (uint32_t)cell[0] + (uint32_t)cell[1] * stride[1] + (uint32_t)cell[2] * stride[2];
         }
     }
-    const uint32_t rx = (uint32_t)g.res[0], rxy = (uint32_t)g.res[0] * (uint32_t)g.res[1];
     uint2 cr_next = make_uint2(0u, 0u);
     bool have_next = false;
     while (__any_sync(kFullMask, active)) {
         uint32_t b = 0, e = 0;
         if (active) {
-            const uint2 cr = have_next ? cr_next
-                                       : __ldg(s.cells + ((uint32_t)cell[0] + (uint32_t)cell[1] * rx +
-                                                          (uint32_t)cell[2] * rxy));
+            const uint2 cr = have_next ? cr_next : __ldg(s.cells + c);
             b = cr.x; e = cr.y;
             if (STATS) h.cells++;
         }
@@ -280,11 +310,10 @@ __device__ void trace_ug(const Scene& s, const G& g, f3 o, f3 d, bool any, Hit& 
             } else {
                 for (int j = 1;; ++j) {
                     float tk;
-                    const bool inside = dda_step(tmax, cell, rcp, g.cs, g.res, &tk);
+                    const bool inside = dda_step(tmax, dt, c, st, left, &tk);
                     active = h.t > tk && inside;
                     if (!active || j >= HR_UG_CELL_STEPS) break;
-                    const uint2 nx =
-                        __ldg(s.cells + ((uint32_t)cell[0] + (uint32_t)cell[1] * rx + (uint32_t)cell[2] * rxy));
+                    const uint2 nx = __ldg(s.cells + c);
                     if (nx.y > nx.x) {
                         cr_next = nx;
                         have_next = true;
@@ -299,37 +328,62 @@ __device__ void trace_ug(const Scene& s, const G& g, f3 o, f3 d, bool any, Hit& 
 
 // Two-level DDA state of one lane (TLGridTraverser.h:79-349).
 struct TL {
-    float rcp[3], tmax[3], tentry;
-    int32_t cell[3];
-    uint32_t lbase, lres[3];   // current top cell: first leaf, sub-grid resolution
-    float scs[3], tm2[3];
-    int32_t c2[3];
+    float rcp[3], tentry;
+    float tmax[3], dt[3];      // top grid: t of the next crossing and its increment per axis
+    uint32_t st[3];            // signed cell strides
+    int32_t left[3];           // steps left inside
+    uint32_t cell;             // current top cell
+    float tm2[3], dt2[3];      // the same of the current top cell's sub-grid
+    uint32_t st2[3];
+    uint32_t left2;            // steps left inside: 10-bit fields, kLeft2Guard | steps
+    uint32_t leaf;             // current leaf
 };
+constexpr uint32_t kLeft2Guard = 0x200u;   // sub-grid resolutions are below 256
+constexpr uint32_t kLeft2Guards = kLeft2Guard | (kLeft2Guard << 10) | (kLeft2Guard << 20);
 
 // Enter the sub-grid of the current top cell at tentry (TLGridTraverser.h:145-197).
 __device__ __forceinline__ void tl_enter(TL& q, const G& g, f3 o, f3 d, uint2 tc) {
-    q.lbase = tc.x;
-    q.lres[0] = tc.y & 0xFFu; q.lres[1] = (tc.y >> 8) & 0xFFu; q.lres[2] = (tc.y >> 16) & 0xFFu;
+    const uint32_t lres[3] = {tc.y & 0xFFu, (tc.y >> 8) & 0xFFu, (tc.y >> 16) & 0xFFu};
+    const uint32_t stride[3] = {1u, lres[0], lres[0] * lres[1]};
     const f3 e2 = mk(o.x + q.tentry * d.x, o.y + q.tentry * d.y, o.z + q.tentry * d.z);
+    q.leaf = tc.x;
+    q.left2 = kLeft2Guards;
 #pragma unroll
     for (int k = 0; k < 3; ++k) {
-        const float cres = (float)q.lres[k];
+        const float cres = (float)lres[k];
         const float srcp = g.rcp[k] * cres;
-        const float mb = (float)q.cell[k] * g.cs[k] + g.bmin[k];
+        const bool fwd = q.rcp[k] > 0.0f;
+        const int32_t cell = fwd ? g.res[k] - 1 - q.left[k] : q.left[k];
+        const float mb = (float)cell * g.cs[k] + g.bmin[k];
         float cf = floorf((comp(e2, k) - mb) * srcp);
         const float scs = 1.0f / srcp;
-        q.scs[k] = scs;
+        q.dt2[k] = scs * fabsf(q.rcp[k]);
         cf = hmin(cres - 1.0f, hmax(cf, 0.0f));
-        const float stp = q.rcp[k] > 0.0f ? 1.0f : 0.0f;
+        const float stp = fwd ? 1.0f : 0.0f;
         q.tm2[k] = ((cf + stp) * scs + mb - comp(o, k)) * q.rcp[k];
-        q.c2[k] = f2i(cf);
+        const uint32_t c2 = (uint32_t)f2i(cf);
+        q.leaf += c2 * stride[k];
+        q.st2[k] = fwd ? stride[k] : 0u - stride[k];
+        q.left2 += (fwd ? lres[k] - 1u - c2 : c2) << (10 * k);
     }
 }
 
+// One step of the sub-grid's DDA (dda_step with the packed step counts).
+__device__ __forceinline__ bool tl_leaf_step(TL& q, float* t_before) {
+    const float a = q.tm2[0], b = q.tm2[1], c = q.tm2[2];
+    const bool ab = a < b;
+    const bool p0 = ab && a < c, p1 = !ab && b < c;
+    *t_before = p0 ? a : (p1 ? b : c);
+    if (p0) { q.tm2[0] = a + q.dt2[0]; q.leaf += q.st2[0]; q.left2 -= 1u; }
+    if (p1) { q.tm2[1] = b + q.dt2[1]; q.leaf += q.st2[1]; q.left2 -= 1u << 10; }
+    if (!(p0 || p1)) { q.tm2[2] = c + q.dt2[2]; q.leaf += q.st2[2]; q.left2 -= 1u << 20; }
+    return (q.left2 & kLeft2Guards) == kLeft2Guards;
+}
+
 // Outer step (TLGridTraverser.h:296-348): returns false when the ray is done.
-__device__ __forceinline__ bool tl_outer_step(TL& q, const G& g, const Hit& h) {
+__device__ __forceinline__ bool tl_outer_step(TL& q, const Hit& h) {
     float tk;
-    const bool inside = dda_step(q.tmax, q.cell, q.rcp, g.cs, g.res, &tk);
+    const bool inside = dda_step(q.tmax, q.dt, q.cell, q.st, q.left, &tk);
     q.tentry = tk;
     return h.t > tk && inside;
 }
@@ -340,9 +394,8 @@ __device__ __forceinline__ bool tl_outer_step(TL& q, const G& g, const Hit& h) {
 // mostly empty cells whose records would miss in L1: the path tracer).
 template <bool STATS, bool OCC = false>
 __device__ __forceinline__ bool tl_seek(TL& q, const Scene& s, const G& g, f3 o, f3 d, Hit& h) {
-    const uint32_t rx = (uint32_t)g.res[0], rxy = (uint32_t)g.res[0] * (uint32_t)g.res[1];
     while (true) {
-        const uint32_t c = (uint32_t)q.cell[0] + (uint32_t)q.cell[1] * rx + (uint32_t)q.cell[2] * rxy;
+        const uint32_t c = q.cell;
         if (STATS) h.cells++;
         bool full = true;
         if (OCC && s.occ) {
@@ -356,13 +409,8 @@ __device__ __forceinline__ bool tl_seek(TL& q, const Scene& s, const G& g, f3 o,
                 return true;
             }
         }
-        if (!tl_outer_step(q, g, h)) return false;
+        if (!tl_outer_step(q, h)) return false;
     }
-}
-
-// index of the current leaf: first leaf of the top cell + x + rx * (y + ry * z)
-__device__ __forceinline__ uint32_t tl_leaf(const TL& q) {
-    return q.lbase + (uint32_t)q.c2[0] + q.lres[0] * (uint32_t)q.c2[1] + q.lres[0] * q.lres[1] * (uint32_t)q.c2[2];
 }
 
 // Inner step (TLGridTraverser.h:225-290): stop when the hit lies before the leaf's exit,
@@ -370,14 +418,13 @@ __device__ __forceinline__ uint32_t tl_leaf(const TL& q) {
 // KL > 1: an empty next leaf (no list to test) is stepped over at once, up to KL leaves.
 template <bool STATS, bool OCC = false, int KL = 1>
 __device__ __forceinline__ bool tl_advance(TL& q, const Scene& s, const G& g, f3 o, f3 d, Hit& h) {
-    const int32_t lres[3] = {(int32_t)q.lres[0], (int32_t)q.lres[1], (int32_t)q.lres[2]};
     for (int j = 1;; ++j) {
         float tk;
-        const bool inside = dda_step(q.tm2, q.c2, q.rcp, q.scs, lres, &tk);
+        const bool inside = tl_leaf_step(q, &tk);
         if (h.t < tk) return false;
-        if (!inside) return tl_outer_step(q, g, h) && tl_seek<STATS, OCC>(q, s, g, o, d, h);
+        if (!inside) return tl_outer_step(q, h) && tl_seek<STATS, OCC>(q, s, g, o, d, h);
         if (j >= KL) return true;
-        const uint2 lr = __ldg(s.leaves + tl_leaf(q));
+        const uint2 lr = __ldg(s.leaves + q.leaf);
         if (lr.y > lr.x) return true;
         if (STATS) h.cells++;
     }
@@ -386,30 +433,41 @@ __device__ __forceinline__ bool tl_advance(TL& q, const Scene& s, const G& g, f3
 // Entry of a ray into the two-level grid (TLGridTraverser.h:79-143): clip to the grid
 // box, the top cell at the entry point, then the first non-empty top cell entered; false
 // if the ray misses the grid or leaves it (or is done) before a non-empty cell.  Per lane.
-template <bool STATS, bool OCC = false>
-__device__ __forceinline__ bool tl_setup(TL& q, const Scene& s, const G& g, f3 o, f3 d, Hit& h) {
+__device__ __forceinline__ bool tl_start(TL& q, const G& g, f3 o, f3 d) {
     q.rcp[0] = 1.0f / d.x; q.rcp[1] = 1.0f / d.y; q.rcp[2] = 1.0f / d.z;
     float t0, t1;
     if (!clip(g, o, q.rcp, &t0, &t1)) return false;
     q.tentry = hmax(0.0f, t0);
     const f3 ep = mk(o.x + q.tentry * d.x, o.y + q.tentry * d.y, o.z + q.tentry * d.z);
+    const uint32_t stride[3] = {1u, (uint32_t)g.res[0], (uint32_t)g.res[0] * (uint32_t)g.res[1]};
+    bool inside = true;
+    q.cell = 0u;
 #pragma unroll
     for (int k = 0; k < 3; ++k) {
         float cf = floorf((comp(ep, k) - g.bmin[k]) * g.rcp[k]);
         cf = hmin((float)g.res[k] - 1.0f, hmax(cf, 0.0f));
-        const float stp = q.rcp[k] > 0.0f ? 1.0f : 0.0f;
+        const bool fwd = q.rcp[k] > 0.0f;
+        const float stp = fwd ? 1.0f : 0.0f;
         q.tmax[k] = ((cf + stp) * g.cs[k] + g.bmin[k] - comp(o, k)) * q.rcp[k];
-        q.cell[k] = f2i(cf);
+        q.dt[k] = g.cs[k] * fabsf(q.rcp[k]);
+        const int32_t cell = f2i(cf);
+        inside = inside && cell < g.res[k] && cell > -1;
+        q.left[k] = fwd ? g.res[k] - 1 - cell : cell;
+        q.st[k] = fwd ? stride[k] : 0u - stride[k];
+        q.cell += (uint32_t)cell * stride[k];
     }
-    if (!(q.cell[0] < g.res[0] && q.cell[0] > -1 && q.cell[1] < g.res[1] && q.cell[1] > -1 &&
-          q.cell[2] < g.res[2] && q.cell[2] > -1))
-        return false;
+    return inside;
+}
+
+template <bool STATS, bool OCC = false>
+__device__ __forceinline__ bool tl_setup(TL& q, const Scene& s, const G& g, f3 o, f3 d, Hit& h) {
+    if (!tl_start(q, g, o, d)) return false;
     return tl_seek<STATS, OCC>(q, s, g, o, d, h);
 }
 
 // a15: two-level DDA, warp-synchronous
 #ifndef HR_RAY_LEAF_STEPS
-#define HR_RAY_LEAF_STEPS 1   // camera and query rays of trace_tl: empty leaves stepped over per warp step
+#define HR_RAY_LEAF_STEPS 4   // camera and query rays of trace_tl: leaves stepped per warp step while they are empty
 #endif
 template <int HM, bool STATS, bool OCC = false>
 __device__ void trace_tl(const Scene& s, const G& g, f3 o, f3 d, bool any, Hit& h, bool active) {
@@ -418,7 +476,7 @@ __device__ void trace_tl(const Scene& s, const G& g, f3 o, f3 d, bool any, Hit& 
     while (__any_sync(kFullMask, active)) {
         uint32_t b = 0, e = 0;
         if (active) {
-            const uint2 lr = __ldg(s.leaves + tl_leaf(q));
+            const uint2 lr = __ldg(s.leaves + q.leaf);
             b = lr.x; e = lr.y;
             if (STATS) h.cells++;
         }
@@ -437,7 +495,7 @@ __device__ void trace_tl(const Scene& s, const G& g, f3 o, f3 d, bool any, Hit& 
 #define HR_PT_SEEK_STEPS 3   // path and shadow rays: empty top cells per warp step (0: unbounded)
 #endif
 #ifndef HR_PT_LEAF_STEPS
-#define HR_PT_LEAF_STEPS 4   // path and shadow rays: leaves stepped per warp step while they are empty
+#define HR_PT_LEAF_STEPS 6   // path and shadow rays: leaves stepped per warp step while they are empty
 #endif
 
 // tl_seek with at most K steps over empty top cells: 1 entered a non-empty cell, 0 done
@@ -445,9 +503,8 @@ __device__ void trace_tl(const Scene& s, const G& g, f3 o, f3 d, bool any, Hit& 
 // looked at (the next call starts there).
 template <bool STATS, bool OCC, int K>
 __device__ __forceinline__ int tl_seek_n(TL& q, const Scene& s, const G& g, f3 o, f3 d, Hit& h) {
-    const uint32_t rx = (uint32_t)g.res[0], rxy = (uint32_t)g.res[0] * (uint32_t)g.res[1];
     for (int i = 0;; ++i) {
-        const uint32_t c = (uint32_t)q.cell[0] + (uint32_t)q.cell[1] * rx + (uint32_t)q.cell[2] * rxy;
+        const uint32_t c = q.cell;
         if (STATS) h.cells++;
         bool full = true;
         if (OCC && s.occ) {
@@ -461,7 +518,7 @@ __device__ __forceinline__ int tl_seek_n(TL& q, const Scene& s, const G& g, f3 o
                 return 1;
             }
         }
-        if (!tl_outer_step(q, g, h)) return 0;
+        if (!tl_outer_step(q, h)) return 0;
         if (i + 1 >= K) return 2;
     }
 }
@@ -469,22 +526,7 @@ __device__ __forceinline__ int tl_seek_n(TL& q, const Scene& s, const G& g, f3 o
 // tl_setup, paced: the lane state after entering the grid
 template <bool STATS, bool OCC, int K>
 __device__ __forceinline__ int tl_setup_n(TL& q, const Scene& s, const G& g, f3 o, f3 d, Hit& h) {
-    q.rcp[0] = 1.0f / d.x; q.rcp[1] = 1.0f / d.y; q.rcp[2] = 1.0f / d.z;
-    float t0, t1;
-    if (!clip(g, o, q.rcp, &t0, &t1)) return 0;
-    q.tentry = hmax(0.0f, t0);
-    const f3 ep = mk(o.x + q.tentry * d.x, o.y + q.tentry * d.y, o.z + q.tentry * d.z);
-#pragma unroll
-    for (int k = 0; k < 3; ++k) {
-        float cf = floorf((comp(ep, k) - g.bmin[k]) * g.rcp[k]);
-        cf = hmin((float)g.res[k] - 1.0f, hmax(cf, 0.0f));
-        const float stp = q.rcp[k] > 0.0f ? 1.0f : 0.0f;
-        q.tmax[k] = ((cf + stp) * g.cs[k] + g.bmin[k] - comp(o, k)) * q.rcp[k];
-        q.cell[k] = f2i(cf);
-    }
-    if (!(q.cell[0] < g.res[0] && q.cell[0] > -1 && q.cell[1] < g.res[1] && q.cell[1] > -1 &&
-          q.cell[2] < g.res[2] && q.cell[2] > -1))
-        return 0;
+    if (!tl_start(q, g, o, d)) return 0;
     return tl_seek_n<STATS, OCC, K>(q, s, g, o, d, h);
 }
 
@@ -494,15 +536,14 @@ template <bool STATS, bool OCC, int K>
 __device__ __forceinline__ int tl_next(TL& q, const Scene& s, const G& g, f3 o, f3 d, Hit& h, int st, bool done) {
     if (st == 1) {
         if (done) return 0;
-        const int32_t lres[3] = {(int32_t)q.lres[0], (int32_t)q.lres[1], (int32_t)q.lres[2]};
         for (int j = 1;; ++j) {
             float tk;
-            const bool inside = dda_step(q.tm2, q.c2, q.rcp, q.scs, lres, &tk);
+            const bool inside = tl_leaf_step(q, &tk);
             if (h.t < tk) return 0;
-            if (!inside) return tl_outer_step(q, g, h) ? tl_seek_n<STATS, OCC, K>(q, s, g, o, d, h) : 0;
+            if (!inside) return tl_outer_step(q, h) ? tl_seek_n<STATS, OCC, K>(q, s, g, o, d, h) : 0;
             if (j >= HR_PT_LEAF_STEPS) return 1;
             // an empty leaf has no list to test: step over it within this warp step
-            const uint2 lr = __ldg(s.leaves + tl_leaf(q));
+            const uint2 lr = __ldg(s.leaves + q.leaf);
             if (lr.y > lr.x) return 1;
             if (STATS) h.cells++;
         }
@@ -519,7 +560,7 @@ __device__ void trace_tl_paced(const Scene& s, const G& g, f3 o, f3 d, bool any,
     while (__any_sync(kFullMask, st != 0)) {
         uint32_t b = 0, e = 0;
         if (st == 1) {
-            const uint2 lr = __ldg(s.leaves + tl_leaf(q));
+            const uint2 lr = __ldg(s.leaves + q.leaf);
             b = lr.x; e = lr.y;
             if (STATS) h.cells++;
         }
