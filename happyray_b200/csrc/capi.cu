@@ -240,8 +240,8 @@ hr_status hr_create(hr_ctx** out, int32_t device, void* stream) {
     }
     for (auto& e : c->ev) cudaEventCreate(&e);
     for (auto& e : c->rev) cudaEventCreate(&e);
-    if (ensure(c, c->counters, 80)) { hr_destroy(c); return HR_ERR_OUT_OF_MEMORY; }   // 8 counter words, 2 pool words
-    cudaMemsetAsync(c->counters.p, 0, 80, c->stream);
+    if (ensure(c, c->counters, 96)) { hr_destroy(c); return HR_ERR_OUT_OF_MEMORY; }   // 8 counter words, 4 pool words
+    cudaMemsetAsync(c->counters.p, 0, 96, c->stream);
     {   // default light: a 0.2 x 0.2 quad at z = 1 centred over (0.5, 0.5), emitting along -z
         const float corner[3] = {0.4f, 0.4f, 1.0f}, e1[3] = {0.2f, 0.0f, 0.0f}, e2[3] = {0.0f, 0.2f, 0.0f};
         const float em = 20.0f;

@@ -177,7 +177,7 @@ __global__ __launch_bounds__(kJobTT, PT ? HR_JOB_PT_MIN_BLOCKS : HR_JOB_MIN_BLOC
                     pend = kNone;
                     next = 0;
                 }
-                if (path_refill(ln, T.cam, tile_local, &next, T.image_id, T.seed, T.fb) == 0u) break;
+                if (path_refill(ln, T.cam, tile_local * 32u, &next, 32u, T.image_id, T.seed, T.fb) == 0u) break;
             }
             if (!__any_sync(kFullMask, ln.has)) break;   // the pool is dry and every path is done
             const bool cont = path_step<kTwoLevel, false, HR_JOB_PT_SEEK_STEPS>(T.s, T.g, T.pk, ln.p, ln.has, n);

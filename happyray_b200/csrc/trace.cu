@@ -23,14 +23,17 @@
 #include <type_traits>
 
 #ifndef HR_AO_REFILL_MIN
-#define HR_AO_REFILL_MIN 12   // idle lanes that make k_ao_samples_tl refill
-#endif
-#ifndef HR_AO_PRIMARY_REFILL_MIN
-#define HR_AO_PRIMARY_REFILL_MIN 32   // idle lanes that make k_ao_primary_tl refill (> 32: k_ao_primary)
+#define HR_AO_REFILL_MIN 12   // idle lanes that make k_ao_samples refill
 #endif
 #ifndef HR_AO_LEAF_STEPS
 #define HR_AO_LEAF_STEPS 6   // AO camera and sample rays: empty leaves stepped over per warp step
 #endif
+// Idle lanes that make a warp of a ray query, or of a shadow-ray query, refill: 1M random
+// closest-hit rays in a 500k-triangle scene at 8 / 20 / 28 / 32 lanes 0.428 / 0.423 / 0.436 /
+// 0.495 ms, shadow rays from its surfaces at 8 / 12 / 16 / 20 1.348 / 1.358 / 1.376 / 1.393;
+// cheap rays (300k in a heightfield of 100k, most of them misses) 0.258 / 0.253 / 0.248 /
+// 0.254, and 0.247 unrefilled with one ray per thread.
+constexpr uint32_t kQueryRefill = 24, kShadowRefill = 12;
 #ifndef HR_TRACE_MIN_BLOCKS
 #define HR_TRACE_MIN_BLOCKS 8   // blocks of kTT per SM the ray kernels' register budget must allow (8: 64 registers)
 #endif
@@ -39,57 +42,77 @@ namespace hr {
 
 namespace {
 
+// The traverser of ray and shadow-ray queries.  Their rays are long and incoherent more
+// often than not, so on a two-level grid they test occupancy bits before cell records and
+// step over up to six empty leaves (1M random rays 0.450 -> 0.428 ms, shadow rays 1.41 ->
+// 1.36); walks over empty top cells paced as the path tracer's measured no better.
+template <int KIND, bool STATS>
+using QueryTrav = std::conditional_t<KIND == kUniform, TravUG<STATS>, TravTL<STATS, true, 0, 6>>;
+
+__device__ __forceinline__ void load_ray(const float* __restrict__ org, const float* __restrict__ dir, uint32_t i, f3& o,
+                                         f3& d) {
+    o = mk(__ldg(org + 3 * (size_t)i), __ldg(org + 3 * (size_t)i + 1), __ldg(org + 3 * (size_t)i + 2));
+    d = mk(__ldg(dir + 3 * (size_t)i), __ldg(dir + 3 * (size_t)i + 1), __ldg(dir + 3 * (size_t)i + 2));
+}
+
+template <bool STATS>
+__device__ __forceinline__ void store_hit(const Scene& s, uint32_t i, f3 o, f3 d, Hit& h, int32_t* __restrict__ oid,
+                                          float* __restrict__ ot, float* __restrict__ ou, float* __restrict__ ov,
+                                          uint32_t* __restrict__ stats) {
+    if (h.hit) refine_uv(s, h.tri, o, d, &h.u, &h.v);
+    oid[i] = h.hit ? (int32_t)h.tri : -1;
+    ot[i] = h.hit ? h.t : FLT_MAX;
+    ou[i] = h.u;
+    ov[i] = h.v;
+    if (STATS) { stats[2 * (size_t)i] = h.cells; stats[2 * (size_t)i + 1] = h.tests; }
+}
+
 template <int KIND, bool STATS>
 __global__ __launch_bounds__(kTT, HR_TRACE_MIN_BLOCKS) void k_trace_rays(Scene s, const float* __restrict__ org, const float* __restrict__ dir,
-                                                    uint32_t n, int32_t* __restrict__ oid, float* __restrict__ ot,
+                                                    RayPool w, int32_t* __restrict__ oid, float* __restrict__ ot,
                                                     float* __restrict__ ou, float* __restrict__ ov,
                                                     uint32_t* __restrict__ stats) {
     const G g = load_g(s.desc);
     gate_scene(s);
-    const uint32_t nl = round32(n);
-    for (uint32_t i = blockIdx.x * kTT + threadIdx.x; i < nl; i += gridDim.x * kTT) {
-        const bool valid = i < n;
-        f3 o = mk(0.0f, 0.0f, 0.0f), d = mk(1.0f, 0.0f, 0.0f);
-        if (valid) {
-            o = mk(__ldg(org + 3 * (size_t)i), __ldg(org + 3 * (size_t)i + 1), __ldg(org + 3 * (size_t)i + 2));
-            d = mk(__ldg(dir + 3 * (size_t)i), __ldg(dir + 3 * (size_t)i + 1), __ldg(dir + 3 * (size_t)i + 2));
-        }
-        Hit h;
-        trace_one<KIND, false, STATS>(s, g, o, d, FLT_MAX, h, valid);
-        if (valid) {
-            if (h.hit) refine_uv(s, h.tri, o, d, &h.u, &h.v);
-            oid[i] = h.hit ? (int32_t)h.tri : -1;
-            ot[i] = h.hit ? h.t : FLT_MAX;
-            ou[i] = h.u;
-            ov[i] = h.v;
-            if (STATS) { stats[2 * (size_t)i] = h.cells; stats[2 * (size_t)i + 1] = h.tests; }
-        }
-    }
+    trace_pool<QueryTrav<KIND, STATS>, kHitClosest, STATS>(
+        s, g, w,
+        [&](uint32_t i, f3& o, f3& d, Hit&) {
+            load_ray(org, dir, i, o, d);
+            return true;
+        },
+        [&](uint32_t i, Hit& h, bool) {
+            f3 o, d;
+            load_ray(org, dir, i, o, d);
+            store_hit<STATS>(s, i, o, d, h, oid, ot, ou, ov, stats);
+        });
+}
+
+// Camera rays by pixel tile, `width` consecutive slots of the tile order per warp and
+// step (grid stride); body(slot) traces the slot's ray with the whole warp, slots past the
+// warp's width or the image are kNoSlot.
+constexpr uint32_t kNoSlot = 0xffffffffu;
+template <class F>
+__device__ __forceinline__ void for_camera_slots(const Cam& cam, uint32_t width, F body) {
+    const uint32_t lane = threadIdx.x & 31u, units = tile_slots(cam) / width;
+    for (uint32_t u = blockIdx.x * (kTT / 32) + (threadIdx.x >> 5); u < units; u += gridDim.x * (kTT / 32))
+        body(lane < width ? u * width + lane : kNoSlot);
 }
 
 template <int KIND, bool STATS>
-__global__ __launch_bounds__(kTT, HR_TRACE_MIN_BLOCKS) void k_trace_primary(Scene s, Cam cam, int32_t* __restrict__ oid,
+__global__ __launch_bounds__(kTT, HR_TRACE_MIN_BLOCKS) void k_trace_primary(Scene s, Cam cam, uint32_t width, int32_t* __restrict__ oid,
                                                        float* __restrict__ ot, float* __restrict__ ou,
                                                        float* __restrict__ ov, uint32_t* __restrict__ stats) {
     const G g = load_g(s.desc);
     gate_scene(s);
-    const uint32_t slots = tile_slots(cam);
     const f3 o = mk(cam.pos[0], cam.pos[1], cam.pos[2]);
-    for (uint32_t slot = blockIdx.x * kTT + threadIdx.x; slot < slots; slot += gridDim.x * kTT) {
-        uint32_t i;
-        const bool valid = tile_pixel(cam, slot, &i);
+    for_camera_slots(cam, width, [&](uint32_t slot) {
+        uint32_t i = 0;
+        const bool valid = slot != kNoSlot && tile_pixel(cam, slot, &i);
         Hit h;
         const f3 d = valid ? primary_dir(cam, i) : mk(1.0f, 0.0f, 0.0f);
         trace_one<KIND, false, STATS>(s, g, o, d, FLT_MAX, h, valid);
-        if (valid) {
-            if (h.hit) refine_uv(s, h.tri, o, d, &h.u, &h.v);
-            oid[i] = h.hit ? (int32_t)h.tri : -1;
-            ot[i] = h.hit ? h.t : FLT_MAX;
-            ou[i] = h.u;
-            ov[i] = h.v;
-            if (STATS) { stats[2 * (size_t)i] = h.cells; stats[2 * (size_t)i + 1] = h.tests; }
-        }
-    }
+        if (valid) store_hit<STATS>(s, i, o, d, h, oid, ot, ou, ov, stats);
+    });
 }
 
 // the ray-file form of render mode 0 (SimpleRayTraverser::integrate,
@@ -97,62 +120,54 @@ __global__ __launch_bounds__(kTT, HR_TRACE_MIN_BLOCKS) void k_trace_primary(Scen
 // pixel i, progressive blend
 template <int KIND>
 __global__ __launch_bounds__(kTT, HR_TRACE_MIN_BLOCKS) void k_render_rays(Scene s, const float* __restrict__ org,
-                                                                     const float* __restrict__ dir, uint32_t n,
+                                                                     const float* __restrict__ dir, RayPool w,
                                                                      int32_t image_id, float* __restrict__ fb,
                                                                      unsigned long long* counter) {
     const G g = load_g(s.desc);
     gate_scene(s);
-    const uint32_t nl = round32(n);
-    for (uint32_t i = blockIdx.x * kTT + threadIdx.x; i < nl; i += gridDim.x * kTT) {
-        const bool valid = i < n;
-        f3 o = mk(0.0f, 0.0f, 0.0f), d = mk(1.0f, 0.0f, 0.0f);
-        if (valid) {
-            o = mk(__ldg(org + 3 * (size_t)i), __ldg(org + 3 * (size_t)i + 1), __ldg(org + 3 * (size_t)i + 2));
-            d = mk(__ldg(dir + 3 * (size_t)i), __ldg(dir + 3 * (size_t)i + 1), __ldg(dir + 3 * (size_t)i + 2));
-        }
-        Hit h;
-        trace_one<KIND, false, false>(s, g, o, d, FLT_MAX, h, valid);
-        if (valid) {
+    uint32_t nrays = 0;
+    trace_pool<QueryTrav<KIND, false>, kHitClosest, false>(
+        s, g, w,
+        [&](uint32_t i, f3& o, f3& d, Hit&) {
+            load_ray(org, dir, i, o, d);
+            return true;
+        },
+        [&](uint32_t i, Hit& h, bool) {
+            f3 o, d;
             float rgb[3];
+            load_ray(org, dir, i, o, d);
             simple_shade(s, h.hit, h.tri, o, d, rgb);
             for (int k = 0; k < 3; ++k) fb[3 * (size_t)i + k] = blend(fb[3 * (size_t)i + k], rgb[k], image_id);
-        }
-        add_rays<false>(counter, false, valid ? 1u : 0u);
-    }
+            nrays += 1;
+        });
+    add_rays<false>(counter, false, nrays);
 }
 
 template <int KIND>
 __global__ __launch_bounds__(kTT, HR_TRACE_MIN_BLOCKS) void k_occluded(Scene s, const float* __restrict__ org, const float* __restrict__ dir,
-                                                  const float* __restrict__ tmax, uint32_t n, uint8_t* __restrict__ occ) {
+                                                  const float* __restrict__ tmax, RayPool w, uint8_t* __restrict__ occ) {
     const G g = load_g(s.desc);
     gate_scene(s);
-    const uint32_t nl = round32(n);
-    for (uint32_t i = blockIdx.x * kTT + threadIdx.x; i < nl; i += gridDim.x * kTT) {
-        const bool valid = i < n;
-        f3 o = mk(0.0f, 0.0f, 0.0f), d = mk(1.0f, 0.0f, 0.0f);
-        float tm = 0.0f;
-        if (valid) {
-            o = mk(org[3 * (size_t)i], org[3 * (size_t)i + 1], org[3 * (size_t)i + 2]);
-            d = mk(dir[3 * (size_t)i], dir[3 * (size_t)i + 1], dir[3 * (size_t)i + 2]);
-            tm = tmax[i];
-        }
-        Hit h;
-        trace_one<KIND, true, false>(s, g, o, d, tm, h, valid);
-        if (valid) occ[i] = h.hit ? 1 : 0;
-    }
+    trace_pool<QueryTrav<KIND, false>, kHitAny, false>(
+        s, g, w,
+        [&](uint32_t i, f3& o, f3& d, Hit& h) {
+            load_ray(org, dir, i, o, d);
+            h.t = __ldg(tmax + i);
+            return true;
+        },
+        [&](uint32_t i, Hit& h, bool) { occ[i] = h.hit ? 1 : 0; });
 }
 
 // mode 0: primary rays with barycentric false colour (SimpleIntegrator.h:41-126)
 template <int KIND, bool STATS>
-__global__ __launch_bounds__(kTT, HR_TRACE_MIN_BLOCKS) void k_render_primary(Scene s, Cam cam, int32_t image_id, uint64_t seed,
+__global__ __launch_bounds__(kTT, HR_TRACE_MIN_BLOCKS) void k_render_primary(Scene s, Cam cam, uint32_t width, int32_t image_id, uint64_t seed,
                                                         float* __restrict__ fb, unsigned long long* counter) {
     const G g = load_g(s.desc);
     gate_scene(s);
-    const uint32_t slots = tile_slots(cam);
     const f3 o = mk(cam.pos[0], cam.pos[1], cam.pos[2]);
-    for (uint32_t slot = blockIdx.x * kTT + threadIdx.x; slot < slots; slot += gridDim.x * kTT) {
-        uint32_t i;
-        const bool valid = tile_pixel(cam, slot, &i);
+    for_camera_slots(cam, width, [&](uint32_t slot) {
+        uint32_t i = 0;
+        const bool valid = slot != kNoSlot && tile_pixel(cam, slot, &i);
         const f3 d = valid ? primary_sample_dir(cam, i, image_id, seed) : mk(1.0f, 0.0f, 0.0f);
         Hit h;
         trace_one<KIND, false, STATS>(s, g, o, d, FLT_MAX, h, valid);
@@ -164,152 +179,66 @@ __global__ __launch_bounds__(kTT, HR_TRACE_MIN_BLOCKS) void k_render_primary(Sce
             fb[3 * (size_t)i + 2] = blend(fb[3 * (size_t)i + 2], rgb[2], image_id);
         }
         add_rays<STATS>(counter, false, valid ? 1u : 0u, h.cells, h.tests);
-    }
+    });
 }
 
 // mode 3, ambient occlusion (AOIntegrator.h:234-351: primary trace, AO rays, shading), as
 // a wavefront of three kernels:
 //   k_ao_primary  camera rays in pixel tiles; misses are shaded at once, hit pixels are
 //                 appended (warp-aggregated) to a queue with their t and triangle;
-//   k_ao_samples  one thread per (hit pixel, sample): AO ray generation as
+//   k_ao_samples  one ray per (hit pixel, sample): AO ray generation as
 //                 RayGenerators.h:286-342 with the configured radius and PCG32 stream of
 //                 the pixel (sample k uses draws 2k and 2k+1), any-hit traversal, and the
 //                 unoccluded count of the pixel (match_any-aggregated atomics);
 //   k_ao_finish   visibility = unoccluded / samples, progressive blend (AOIntegrator.h:168-175).
 template <int KIND, bool STATS>
-__global__ __launch_bounds__(kTT, HR_TRACE_MIN_BLOCKS) void k_ao_primary(Scene s, Cam cam, int32_t image_id, float* __restrict__ fb,
-                                                    float* __restrict__ hit_t, uint32_t* __restrict__ hit_tri,
-                                                    uint32_t* __restrict__ unocc, uint32_t* __restrict__ queue,
-                                                    uint32_t* qcount, unsigned long long* counter) {
-    const G g = load_g(s.desc);
-    gate_scene(s);
-    const uint32_t slots = tile_slots(cam);
-    const f3 o = mk(cam.pos[0], cam.pos[1], cam.pos[2]);
-    const uint32_t lane = threadIdx.x & 31u, lt = (1u << lane) - 1u;
-    for (uint32_t slot = blockIdx.x * kTT + threadIdx.x; slot < slots; slot += gridDim.x * kTT) {
-        uint32_t pix;
-        const bool valid = tile_pixel(cam, slot, &pix);
-        Hit h;
-        trace_one<KIND, false, STATS>(s, g, o, valid ? primary_dir(cam, pix) : mk(1.0f, 0.0f, 0.0f), FLT_MAX, h, valid);
-        const bool hit = valid && h.hit;
-        if (hit) {
-            hit_t[pix] = h.t;
-            hit_tri[pix] = h.tri;
-            unocc[pix] = 0u;
-        } else if (valid) {
-            const float val = blend(fb[3 * (size_t)pix], 1.0f, image_id);
-            fb[3 * (size_t)pix] = val;
-            fb[3 * (size_t)pix + 1] = val;
-            fb[3 * (size_t)pix + 2] = val;
-        }
-        const uint32_t m = __ballot_sync(kFullMask, hit);
-        if (m) {
-            const int leader = __ffs(m) - 1;
-            uint32_t base = 0;
-            if ((int)lane == leader) base = atomicAdd(qcount, (uint32_t)__popc(m));
-            base = __shfl_sync(kFullMask, base, leader);
-            if (hit) queue[base + __popc(m & lt)] = pix;
-        }
-        add_rays<STATS>(counter, false, valid ? 1u : 0u, h.cells, h.tests);
-    }
-}
+using AoTrav = std::conditional_t<KIND == kUniform, TravUG<STATS>, TravTL<STATS, false, 0, HR_AO_LEAF_STEPS>>;
 
+// AO camera rays, with lanes refilled inside the traversal loop: once
+// all `width` lanes a warp uses are done (their pixels shaded or queued), they take that
+// many consecutive pixel slots of the tile order from the pool.
 template <int KIND, bool STATS>
-__global__ __launch_bounds__(kTT, HR_TRACE_MIN_BLOCKS) void k_ao_samples(Scene s, Cam cam, int32_t spp, float alpha_frac, float alpha_abs,
-                                                    uint64_t seed, int32_t image_id, const float* __restrict__ hit_t,
-                                                    const uint32_t* __restrict__ hit_tri,
-                                                    const uint32_t* __restrict__ queue, const uint32_t* qcount,
-                                                    uint32_t* __restrict__ unocc, unsigned long long* counter) {
-    const G g = load_g(s.desc);
-    gate_scene(s);
-    float alpha = alpha_abs;
-    if (!(alpha > 0.0f)) {
-        const f3 dd = mk(g.bmax[0] - g.bmin[0], g.bmax[1] - g.bmin[1], g.bmax[2] - g.bmin[2]);
-        alpha = alpha_frac * sqrtf(dot(dd, dd));
-    }
-    const float off = 0.01f * alpha;
-    const f3 o = mk(cam.pos[0], cam.pos[1], cam.pos[2]);
-    const uint32_t nitems = *qcount * (uint32_t)spp;
-    const uint32_t nloop = round32(nitems);
-    for (uint32_t item = blockIdx.x * kTT + threadIdx.x; item < nloop; item += gridDim.x * kTT) {
-        const bool valid = item < nitems;
-        uint32_t pix = 0xffffffffu;
-        f3 ao = mk(0.0f, 0.0f, 0.0f), w = mk(1.0f, 0.0f, 0.0f);
-        if (valid) {
-            const uint32_t q = item / (uint32_t)spp, k = item % (uint32_t)spp;
-            pix = queue[q];
-            const f3 d = primary_dir(cam, pix);
-            const float t = hit_t[pix];
-            const f3 p = mk(o.x + t * d.x, o.y + t * d.y, o.z + t * d.z);
-            const f3 nrm = face_normal(s, hit_tri[pix], d);
-            Pcg32 rng;
-            pcg_seed(rng, ((uint64_t)(uint32_t)image_id << 32) | pix, seed);
-            pcg_skip_pairs(rng, k);
-            const float u1 = pcg_float(rng), u2 = pcg_float(rng);
-            w = cosine_dir(nrm, u1, u2);
-            ao = mk(p.x + off * w.x, p.y + off * w.y, p.z + off * w.z);
-        }
-        Hit hs;
-        trace_one<KIND, true, STATS>(s, g, ao, w, alpha, hs, valid);
-        const bool free = valid && !hs.hit;
-        const uint32_t peers = __match_any_sync(kFullMask, pix);
-        const uint32_t nfree = __popc(__ballot_sync(kFullMask, free) & peers);
-        if (valid && nfree && (int)(threadIdx.x & 31u) == __ffs(peers) - 1) atomicAdd(unocc + pix, nfree);
-        add_rays<STATS>(counter, true, valid ? 1u : 0u, hs.cells, hs.tests);
-    }
-}
-
-// AO camera rays on a two-level grid with lanes refilled inside the traversal loop: once
-// HR_AO_PRIMARY_REFILL_MIN lanes are done (their pixels shaded or queued as k_ao_primary
-// does), they take that many consecutive pixel slots of the tile order from the pool.
-template <bool STATS>
-__global__ __launch_bounds__(kTT, HR_TRACE_MIN_BLOCKS) void k_ao_primary_tl(Scene s, Cam cam, int32_t image_id,
+__global__ __launch_bounds__(kTT, HR_TRACE_MIN_BLOCKS) void k_ao_primary(Scene s, Cam cam, int32_t image_id,
                                                               float* __restrict__ fb, float* __restrict__ hit_t,
                                                               uint32_t* __restrict__ hit_tri, uint32_t* __restrict__ unocc,
                                                               uint32_t* __restrict__ queue, uint32_t* qcount,
-                                                              unsigned long long* counter, uint32_t* work) {
+                                                              unsigned long long* counter, uint32_t* work, uint32_t width) {
     const G g = load_g(s.desc);
     gate_scene(s);
     const uint32_t slots = tile_slots(cam);
     const f3 o = mk(cam.pos[0], cam.pos[1], cam.pos[2]);
     const uint32_t lane = threadIdx.x & 31u, lt = (1u << lane) - 1u;
-    TL q;
+    AoTrav<KIND, STATS> q;
+    q.st = 0;
     Hit h;
     h.t = FLT_MAX; h.u = 0.0f; h.v = 0.0f; h.tri = 0; h.hit = false; h.cells = 0; h.tests = 0;
     f3 d = mk(1.0f, 0.0f, 0.0f);
     uint32_t pix = 0, nrays = 0, ncells = 0, ntests = 0;
-    bool has = false, valid = false, active = false, dry = false;
+    bool has = false, valid = false, dry = false;
     while (true) {
-        const uint32_t need = __ballot_sync(kFullMask, !has);
-        if (need && !dry && (__popc(need) >= HR_AO_PRIMARY_REFILL_MIN || need == kFullMask ||
-                             !__any_sync(kFullMask, active))) {   // warp-uniform
+        const uint32_t need = __ballot_sync(kFullMask, !has && lane < width);
+        if (!dry && ((uint32_t)__popc(need) == width || (need && !__any_sync(kFullMask, q.st != 0)))) {   // warp-uniform
             const int leader = __ffs(need) - 1;
             uint32_t base = 0;
             if ((int)lane == leader) base = atomicAdd(work, (uint32_t)__popc(need));
             base = __shfl_sync(kFullMask, base, leader);
             if (base + (uint32_t)__popc(need) >= slots) dry = true;
             const uint32_t slot = base + __popc(need & lt);
-            if (!has && slot < slots) {
+            if (((need >> lane) & 1u) && slot < slots) {
                 has = true;
                 valid = tile_pixel(cam, slot, &pix);
                 h.t = FLT_MAX; h.u = 0.0f; h.v = 0.0f; h.tri = 0; h.hit = false; h.cells = 0; h.tests = 0;
-                active = false;
                 if (valid) {
                     d = primary_dir(cam, pix);
-                    if (s.ntri != 0u) active = tl_setup<STATS>(q, s, g, o, d, h);
+                    if (s.ntri != 0u) q.start(s, g, o, d, h);
                 }
             }
         }
         if (!__any_sync(kFullMask, has)) break;   // the pool is dry and no ray is in flight
-        uint32_t b = 0, e = 0;
-        if (active) {
-            const uint2 lr = __ldg(s.leaves + q.leaf);
-            b = lr.x; e = lr.y;
-            if (STATS) h.cells++;
-        }
-        const bool done = test_lists<kHitClosest, STATS>(s, o, d, b, e, false, h);
-        if (active) active = !done && tl_advance<STATS, false, HR_AO_LEAF_STEPS>(q, s, g, o, d, h);
-        const bool fin = has && !active;
+        const uint2 r = q.range(s, h);
+        const bool done = test_lists<kHitClosest, STATS>(s, o, d, r.x, r.y, false, h);
+        q.next(s, g, o, d, h, done);
+        const bool fin = has && q.st == 0;
         const bool hit = fin && valid && h.hit;
         if (hit) {
             hit_t[pix] = h.t;
@@ -341,15 +270,14 @@ __global__ __launch_bounds__(kTT, HR_TRACE_MIN_BLOCKS) void k_ao_primary_tl(Scen
     add_rays<STATS>(counter, false, nrays, ncells, ntests);
 }
 
-// AO samples on a two-level grid with lanes refilled inside the traversal loop: a lane
+// AO samples, with lanes refilled inside the traversal loop: a lane
 // whose ray is done (occluded, or out of the grid or past the radius) retires it and
 // waits; once HR_AO_REFILL_MIN lanes wait (or no ray is left in flight) they take the next
 // (hit pixel, sample) items from the pool together, so a warp keeps most of its lanes
 // busy until the pool runs dry instead of waiting for its longest ray, and the divergent
-// ray set-up runs for many lanes at once.  Per ray the generation, traversal and result
-// are those of k_ao_samples.
-template <bool STATS>
-__global__ __launch_bounds__(kTT, HR_TRACE_MIN_BLOCKS) void k_ao_samples_tl(Scene s, Cam cam, int32_t spp, float alpha_frac,
+// ray set-up runs for many lanes at once.
+template <int KIND, bool STATS>
+__global__ __launch_bounds__(kTT, HR_TRACE_MIN_BLOCKS) void k_ao_samples(Scene s, Cam cam, int32_t spp, float alpha_frac,
                                                               float alpha_abs, uint64_t seed, int32_t image_id,
                                                               const float* __restrict__ hit_t,
                                                               const uint32_t* __restrict__ hit_tri,
@@ -367,23 +295,27 @@ __global__ __launch_bounds__(kTT, HR_TRACE_MIN_BLOCKS) void k_ao_samples_tl(Scen
     const f3 cpos = mk(cam.pos[0], cam.pos[1], cam.pos[2]);
     const uint32_t nitems = *qcount * (uint32_t)spp;
     const uint32_t lane = threadIdx.x & 31u, lt = (1u << lane) - 1u;
-    TL q;
+    // rays a warp holds at a time (as ray_width): fewer where the items would not fill the warps
+    uint32_t width = 32u;
+    while (width > 1u && nitems < gridDim.x * (kTT / 32u) * width) width /= 2u;
+    AoTrav<KIND, STATS> q;
+    q.st = 0;
     Hit h;
     h.t = alpha; h.u = 0.0f; h.v = 0.0f; h.tri = 0; h.hit = false; h.cells = 0; h.tests = 0;
     f3 o = mk(0.0f, 0.0f, 0.0f), w = mk(1.0f, 0.0f, 0.0f);
     uint32_t pix = 0xffffffffu, nrays = 0, ncells = 0, ntests = 0;
-    bool has = false, active = false, dry = s.ntri == 0u;
+    bool has = false, dry = s.ntri == 0u;
     while (true) {
-        const uint32_t need = __ballot_sync(kFullMask, !has);
-        if (need && !dry && (__popc(need) >= HR_AO_REFILL_MIN || need == kFullMask ||
-                             !__any_sync(kFullMask, active))) {   // warp-uniform
+        const uint32_t need = __ballot_sync(kFullMask, !has && lane < width);
+        if (need && !dry && (__popc(need) >= HR_AO_REFILL_MIN ||
+                             !__any_sync(kFullMask, q.st != 0))) {   // warp-uniform
             const int leader = __ffs(need) - 1;
             uint32_t base = 0;
             if ((int)lane == leader) base = atomicAdd(work, (uint32_t)__popc(need));
             base = __shfl_sync(kFullMask, base, leader);
             if (base + (uint32_t)__popc(need) >= nitems) dry = true;
             const uint32_t item = base + __popc(need & lt);
-            if (!has && item < nitems) {
+            if (((need >> lane) & 1u) && item < nitems) {
                 has = true;
                 const uint32_t qi = item / (uint32_t)spp, k = item % (uint32_t)spp;
                 pix = queue[qi];
@@ -398,19 +330,14 @@ __global__ __launch_bounds__(kTT, HR_TRACE_MIN_BLOCKS) void k_ao_samples_tl(Scen
                 w = cosine_dir(nrm, u1, u2);
                 o = mk(p.x + off * w.x, p.y + off * w.y, p.z + off * w.z);
                 h.t = alpha; h.hit = false; h.cells = 0; h.tests = 0;
-                active = tl_setup<STATS>(q, s, g, o, w, h);
+                q.start(s, g, o, w, h);
             }
         }
         if (!__any_sync(kFullMask, has)) break;   // the pool is dry and no ray is in flight
-        uint32_t b = 0, e = 0;
-        if (active) {
-            const uint2 lr = __ldg(s.leaves + q.leaf);
-            b = lr.x; e = lr.y;
-            if (STATS) h.cells++;
-        }
-        const bool done = test_lists<kHitAny, STATS>(s, o, w, b, e, true, h);
-        if (active) active = !done && tl_advance<STATS, false, HR_AO_LEAF_STEPS>(q, s, g, o, w, h);
-        const bool fin = has && !active;
+        const uint2 r = q.range(s, h);
+        const bool done = test_lists<kHitAny, STATS>(s, o, w, r.x, r.y, true, h);
+        q.next(s, g, o, w, h, done);
+        const bool fin = has && q.st == 0;
         const uint32_t peers = __match_any_sync(kFullMask, fin ? pix : 0xffffffffu);
         const uint32_t nfree = __popc(__ballot_sync(kFullMask, fin && !h.hit) & peers);
         if (fin && nfree && (int)lane == __ffs(peers) - 1) atomicAdd(unocc + pix, nfree);
@@ -437,9 +364,6 @@ __global__ void k_ao_finish(const uint32_t* __restrict__ queue, const uint32_t* 
     }
 }
 
-#ifndef HR_AO_REFILL
-#define HR_AO_REFILL 1   // two-level AO samples by k_ao_samples_tl (lanes refilled in the traversal loop)
-#endif
 #ifndef HR_PT_SMEM_STATE
 #define HR_PT_SMEM_STATE 1   // path state in shared memory (registers left to the traversal)
 #endif
@@ -455,11 +379,11 @@ template <int KIND, bool STATS>
 __global__ __launch_bounds__(kTT, HR_PT_MIN_BLOCKS) void k_render_pt(Scene s, Cam cam, const LightSet* __restrict__ ls, int32_t bounces,
                                                                   float albedo, float eps_frac, uint64_t seed,
                                                                   int32_t image_id, float* __restrict__ fb,
-                                                                  unsigned long long* counter, uint32_t* work) {
+                                                                  unsigned long long* counter, uint32_t* work, uint32_t width) {
     const G g = load_g(s.desc);
     gate_scene(s);
     const PtConsts k = pt_consts(g, ls, bounces, albedo, eps_frac);
-    const uint32_t ntiles = tile_slots(cam) >> 5;
+    const uint32_t nunits = tile_slots(cam) / width;   // a warp takes `width` pixel slots at a time
     const uint32_t lane = threadIdx.x & 31u;
 #if HR_PT_SMEM_STATE
     // the path state lives in shared memory, so the traversal has the registers to itself
@@ -473,22 +397,22 @@ __global__ __launch_bounds__(kTT, HR_PT_MIN_BLOCKS) void k_render_pt(Scene s, Ca
     PathLane ln;
 #endif
     PtCounts n;
-    uint32_t tile = 0, next = 32u;
+    uint32_t slot0 = 0, next = width;
     bool more = true;
     while (true) {
         while (more) {
-            if (next >= 32u) {
+            if (next >= width) {
                 uint32_t t = 0;
                 if (lane == 0) t = atomicAdd(work, 1u);
                 t = __shfl_sync(kFullMask, t, 0);
-                if (t >= ntiles) {
+                if (t >= nunits) {
                     more = false;
                     break;
                 }
-                tile = t;
+                slot0 = t * width;
                 next = 0;
             }
-            if (path_refill(ln, cam, tile, &next, image_id, seed, fb) == 0u) break;
+            if (path_refill(ln, cam, slot0, &next, width, image_id, seed, fb) == 0u) break;
         }
         if (!__any_sync(kFullMask, ln.has)) break;
         const bool cont = path_step<KIND, STATS>(s, g, k, ln.p, ln.has, n);
@@ -525,6 +449,42 @@ Cam make_cam(const hr_ctx* c) {
     return k;
 }
 
+// Rays a warp holds at a time when n rays are shared out to `warps` resident warps: 32, or
+// a smaller power of two (at least `least`) while n rays would not fill them `waves` times.
+// A warp step costs the longest of its lanes' walks, and a small launch is as long as its
+// slowest warp: with fewer rays per warp the walks are shorter, a ray's list is still
+// tested by all 32 lanes, and the GPU's other warps take the rest.
+uint32_t ray_width(uint64_t n, uint64_t warps, uint32_t waves, uint32_t least) {
+    uint32_t w = 32u;
+    while (w > least && n < warps * w * waves) w /= 2u;
+    return w;
+}
+
+// Camera rays: warps filled four times over, at least 4 rays each (coherent rays share their
+// walk, and the short launches' tail is a tile over dense cells).  Per ms at 32 / 16 / 8 / 4
+// rays: 256 x 256 uniform heightfield 0.067 / 0.061 / 0.054 / 0.051, 640 x 480 two-level
+// 100k 0.157 / 0.149 / 0.166 / 0.227, 801 x 601 uniform grid with lists of thousands 2.56 /
+// 1.45 / 1.34 / 1.68, 1080p two-level 1M 0.586 / 0.779 / 1.29 / 2.14.
+uint32_t camera_width(const hr_ctx* c) {
+    const uint64_t slots = (((uint64_t)c->cam.w + 7u) / 8u) * (((uint64_t)c->cam.h + 3u) / 4u) * 32u;
+    return ray_width(slots, (uint64_t)c->num_sms * HR_TRACE_MIN_BLOCKS * (kTT / 32), 4, 4);
+}
+
+// The pool of a ray query over n rays and its block count (blocks resident at once; the
+// launch bounds allow HR_TRACE_MIN_BLOCKS per SM).  A query that fits takes the fewest rays
+// per warp that still have all of them in flight at once (64 rays 0.044 -> 0.028 ms, 4096
+// rays in a 2M-triangle scene 0.130 -> 0.091); a larger one refills from the pool.
+void ray_pool(const hr_ctx* c, uint32_t n, uint32_t refill, RayPool* w, int* blocks) {
+    const uint64_t wpb = kTT / 32, warps = (uint64_t)c->num_sms * HR_TRACE_MIN_BLOCKS * wpb;
+    w->n = n;
+    w->width = 32u;
+    while (w->width > 1u && n <= warps * (w->width / 2u)) w->width /= 2u;
+    w->refill = std::min(refill, w->width);
+    const uint64_t want = ((uint64_t)n + w->width - 1) / w->width;   // warps
+    *blocks = (int)((std::min(want, warps) + wpb - 1) / wpb);
+    w->next = want > (uint64_t)*blocks * wpb ? c->counters.as<unsigned long long>() + 9 : nullptr;
+}
+
 int grid_for(const hr_ctx* c, uint32_t n) {
     uint32_t b = (n + kTT - 1) / kTT;
     uint32_t cap = (uint32_t)c->num_sms * 16u;
@@ -556,9 +516,12 @@ int launch_trace_rays(hr_ctx* c, const float* org, const float* dir, uint32_t n,
                       float* v, uint32_t* stats) {
     if (n == 0) return 0;
     Scene s = make_scene(c);
+    RayPool w;
+    int nb;
+    ray_pool(c, n, kQueryRefill, &w, &nb);
     c->launches += 1;
     by_kind(s.kind, stats != nullptr, [&](auto K, auto S) {
-        k_trace_rays<K(), S()><<<grid_for(c, n), kTT, 0, c->stream>>>(s, org, dir, n, id, t, u, v, stats);
+        k_trace_rays<K(), S()><<<nb, kTT, 0, c->stream>>>(s, org, dir, w, id, t, u, v, stats);
     });
     return cuda_check(c, cudaGetLastError(), "trace_rays launch");
 }
@@ -569,29 +532,36 @@ int launch_trace_primary(hr_ctx* c, int32_t* id, float* t, float* u, float* v, u
     const uint32_t n = (uint32_t)k.w * (uint32_t)k.h;
     if (n == 0) return 0;
     c->launches += 1;
-    const int gb = grid_for(c, slots_for(c));
+    const uint32_t width = camera_width(c);
     by_kind(s.kind, stats != nullptr, [&](auto K, auto S) {
-        k_trace_primary<K(), S()><<<gb, kTT, 0, c->stream>>>(s, k, id, t, u, v, stats);
+        k_trace_primary<K(), S()><<<grid_for(c, slots_for(c) / width * 32u), kTT, 0, c->stream>>>(s, k, width, id, t, u, v,
+                                                                                                 stats);
     });
     return cuda_check(c, cudaGetLastError(), "trace_primary launch");
 }
 
 int launch_render_rays(hr_ctx* c, const float* org, const float* dir, uint32_t n, int32_t image_id, float* fb) {
     if (n == 0) return 0;
+    RayPool w;
+    int nb;
+    ray_pool(c, n, kQueryRefill, &w, &nb);
     c->launches += 1;
     const Scene s = make_scene(c);
     unsigned long long* ctr = c->counters.as<unsigned long long>();
     by_kind(s.kind, false, [&](auto K, auto) {
-        k_render_rays<K()><<<grid_for(c, n), kTT, 0, c->stream>>>(s, org, dir, n, image_id, fb, ctr);
+        k_render_rays<K()><<<nb, kTT, 0, c->stream>>>(s, org, dir, w, image_id, fb, ctr);
     });
     return cuda_check(c, cudaGetLastError(), "render_rays launch");
 }
 
 int launch_occluded(hr_ctx* c, const float* org, const float* dir, const float* tmax, uint32_t n, uint8_t* occ) {
     if (n == 0) return 0;
+    RayPool w;
+    int nb;
+    ray_pool(c, n, kShadowRefill, &w, &nb);
     c->launches += 1;
     const Scene s = make_scene(c);
-    by_kind(s.kind, false, [&](auto K, auto) { k_occluded<K()><<<grid_for(c, n), kTT, 0, c->stream>>>(s, org, dir, tmax, n, occ); });
+    by_kind(s.kind, false, [&](auto K, auto) { k_occluded<K()><<<nb, kTT, 0, c->stream>>>(s, org, dir, tmax, w, occ); });
     return cuda_check(c, cudaGetLastError(), "occluded launch");
 }
 
@@ -601,19 +571,21 @@ int launch_render(hr_ctx* c, int32_t mode, int32_t image_id, float* d_fb) {
     const uint32_t n = (uint32_t)k.w * (uint32_t)k.h;
     if (n == 0) return 0;
     unsigned long long* ctr = c->counters.as<unsigned long long>();
-    const int gb = grid_for(c, slots_for(c));
     const bool st = c->collect_stats;
     cudaStream_t strm = c->stream;
     auto mark = [&](int i) { if (c->timing && i < 8) cudaEventRecord(c->rev[i], strm); };
     c->nrender_ev = 0;
     switch (mode) {
-    case 0:
+    case 0: {
+        const uint32_t width = camera_width(c);
+        const int gw = grid_for(c, slots_for(c) / width * 32u);
         c->launches += 1;
         mark(0);
-        by_kind(s.kind, st, [&](auto K, auto S) { k_render_primary<K(), S()><<<gb, kTT, 0, strm>>>(s, k, image_id, c->ip.seed, d_fb, ctr); });
+        by_kind(s.kind, st, [&](auto K, auto S) { k_render_primary<K(), S()><<<gw, kTT, 0, strm>>>(s, k, width, image_id, c->ip.seed, d_fb, ctr); });
         mark(1);
         c->nrender_ev = 2;
         break;
+    }
     case 1:
     case 2: {
         const LightSet* l = c->lights_dev.as<LightSet>();
@@ -628,9 +600,11 @@ int launch_render(hr_ctx* c, int32_t mode, int32_t image_id, float* d_fb) {
                 cudaGetLastError();
                 nb = 1;
             }
-            const int gp = std::min(gb, nb * c->num_sms);
+            const uint32_t width = ray_width(slots_for(c), (uint64_t)nb * c->num_sms * (kTT / 32), 1, 1);
+            const uint32_t need = (slots_for(c) / width + kTT / 32 - 1) / (kTT / 32);   // blocks
+            const int gp = (int)std::min(need, (uint32_t)(nb * c->num_sms));
             k_render_pt<K(), S()><<<gp, kTT, 0, strm>>>(s, k, l, c->ip.pt_bounces, c->ip.albedo, c->ip.ray_eps_frac,
-                                                        c->ip.seed, image_id, d_fb, ctr, work);
+                                                        c->ip.seed, image_id, d_fb, ctr, work, width);
         });
         mark(1);
         c->nrender_ev = 2;
@@ -647,43 +621,19 @@ int launch_render(hr_ctx* c, int32_t mode, int32_t image_id, float* d_fb) {
         const int spp = c->ip.ao_samples;
         c->launches += 3;
         mark(0);
+        // blocks of both kernels: all resident at once (the launch bounds allow HR_TRACE_MIN_BLOCKS per SM)
+        const int nb = HR_TRACE_MIN_BLOCKS * c->num_sms;
+        const uint32_t width = camera_width(c);
         by_kind(s.kind, st, [&](auto K, auto S) {
-            if (HR_AO_PRIMARY_REFILL_MIN <= 32 && K() == kTwoLevel) {
-                int nb = 0;
-                if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, k_ao_primary_tl<S()>, kTT, 0) != cudaSuccess ||
-                    nb < 1) {
-                    cudaGetLastError();
-                    nb = 1;
-                }
-                k_ao_primary_tl<S()><<<std::min(gb, nb * c->num_sms), kTT, 0, strm>>>(
-                    s, k, image_id, d_fb, c->hit_t.as<float>(), c->hit_tri.as<uint32_t>(), c->unocc.as<uint32_t>(),
-                    c->queue.as<uint32_t>(), qcount, ctr, qcount + 2);
-            } else {
-                k_ao_primary<K(), S()><<<gb, kTT, 0, strm>>>(s, k, image_id, d_fb, c->hit_t.as<float>(),
-                                                             c->hit_tri.as<uint32_t>(), c->unocc.as<uint32_t>(),
-                                                             c->queue.as<uint32_t>(), qcount, ctr);
-            }
+            k_ao_primary<K(), S()><<<std::min(grid_for(c, slots_for(c) / width * 32u), nb), kTT, 0, strm>>>(
+                s, k, image_id, d_fb, c->hit_t.as<float>(), c->hit_tri.as<uint32_t>(), c->unocc.as<uint32_t>(),
+                c->queue.as<uint32_t>(), qcount, ctr, qcount + 2, width);
         });
         mark(1);
-        const int gs = c->num_sms * 16;
         by_kind(s.kind, st, [&](auto K, auto S) {
-            if (HR_AO_REFILL && K() == kTwoLevel) {
-                int nb = 0;
-                if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, k_ao_samples_tl<S()>, kTT, 0) != cudaSuccess ||
-                    nb < 1) {
-                    cudaGetLastError();
-                    nb = 1;
-                }
-                k_ao_samples_tl<S()><<<nb * c->num_sms, kTT, 0, strm>>>(
-                    s, k, spp, c->ip.ao_radius_frac, c->ip.ao_radius_abs, c->ip.seed, image_id, c->hit_t.as<float>(),
-                    c->hit_tri.as<uint32_t>(), c->queue.as<uint32_t>(), qcount, c->unocc.as<uint32_t>(), ctr,
-                    qcount + 1);
-            } else {
-                k_ao_samples<K(), S()><<<gs, kTT, 0, strm>>>(s, k, spp, c->ip.ao_radius_frac, c->ip.ao_radius_abs,
-                                                             c->ip.seed, image_id, c->hit_t.as<float>(),
-                                                             c->hit_tri.as<uint32_t>(), c->queue.as<uint32_t>(), qcount,
-                                                             c->unocc.as<uint32_t>(), ctr);
-            }
+            k_ao_samples<K(), S()><<<nb, kTT, 0, strm>>>(
+                s, k, spp, c->ip.ao_radius_frac, c->ip.ao_radius_abs, c->ip.seed, image_id, c->hit_t.as<float>(),
+                c->hit_tri.as<uint32_t>(), c->queue.as<uint32_t>(), qcount, c->unocc.as<uint32_t>(), ctr, qcount + 1);
         });
         mark(2);
         k_ao_finish<<<c->num_sms * 4, 256, 0, strm>>>(c->queue.as<uint32_t>(), qcount, c->unocc.as<uint32_t>(), spp,

@@ -19,6 +19,8 @@
 #include "hr_internal.h"
 #include "hr_block.cuh"
 
+#include <type_traits>
+
 namespace hr {
 namespace {
 
@@ -250,81 +252,88 @@ __device__ __forceinline__ bool clip(const G& g, f3 o, const float* rcp, float* 
     return *t1 > *t0 && *t1 >= 0.0f;
 }
 
-// a14: uniform grid DDA (UGridTraverser.h:76-172), warp-synchronous.  After a lane's list
-// test it steps on over up to HR_UG_CELL_STEPS - 1 empty cells within the same warp step
-// (an empty cell has no list to test) and keeps the range of the non-empty cell it stops
-// at for the next step; each lane visits the same cells in the same order as one cell per
-// step would.
+// A traverser holds one lane's walk through a grid: start() enters the grid, range() is the
+// list of the current cell, next() moves on after that list was tested.  st is 0 once the
+// ray is done, 1 while it stands in a cell or leaf whose list is to be tested, and 2 while
+// a paced two-level walk crosses empty top cells (no list).
+
+// a14: uniform grid DDA (UGridTraverser.h:76-172).  After its list test a lane steps on
+// over up to HR_UG_CELL_STEPS - 1 empty cells within the same warp step (an empty cell has
+// no list to test) and keeps the range of the non-empty cell it stops at for the next
+// step; each lane visits the same cells in the same order as one cell per step would.
 #ifndef HR_UG_CELL_STEPS
 #define HR_UG_CELL_STEPS 4
 #endif
-template <int HM, bool STATS>
-__device__ void trace_ug(const Scene& s, const G& g, f3 o, f3 d, bool any, Hit& h, bool active) {
-    float tmax[3] = {0.0f, 0.0f, 0.0f}, dt[3] = {0.0f, 0.0f, 0.0f};
-    int32_t left[3] = {0, 0, 0};
-    uint32_t st[3] = {0u, 0u, 0u};
-    uint32_t c = 0;   // current cell
-    if (active) {
+template <bool STATS>
+struct TravUG {
+    float tmax[3], dt[3];      // t of the next crossing and its increment per axis
+    int32_t left[3];           // steps left inside
+    uint32_t st3[3];           // signed cell strides
+    uint32_t cell;
+    uint2 cr_next;             // range of the current cell, if have_next
+    bool have_next;
+    int st;
+
+    __device__ __forceinline__ void start(const Scene& s, const G& g, f3 o, f3 d, Hit& h) {
+        st = 0;
+        have_next = false;
         const float rcp[3] = {1.0f / d.x, 1.0f / d.y, 1.0f / d.z};
         float t0, t1;
-        active = clip(g, o, rcp, &t0, &t1);
-        if (active) {
-            f3 ep = o;
-            if (t0 >= 0.0f) {
-                const float te = t0 + kEps;
-                ep = mk(o.x + te * d.x, o.y + te * d.y, o.z + te * d.z);
-            }
-            int32_t cell[3];
-            const uint32_t stride[3] = {1u, (uint32_t)g.res[0], (uint32_t)g.res[0] * (uint32_t)g.res[1]};
-#pragma unroll
-            for (int k = 0; k < 3; ++k) {
-                float cf = floorf((comp(ep, k) - g.bmin[k]) * g.rcp[k]);
-                cf = hmin((float)g.res[k] - 1.0f, hmax(cf, 0.0f));
-                const bool fwd = rcp[k] > 0.0f;
-                const float stp = fwd ? 1.0f : 0.0f;
-                tmax[k] = ((cf + stp) * g.cs[k] + g.bmin[k] - comp(o, k)) * rcp[k];
-                dt[k] = g.cs[k] * fabsf(rcp[k]);
-                cell[k] = f2i(cf);
-                left[k] = fwd ? g.res[k] - 1 - cell[k] : cell[k];
-                st[k] = fwd ? stride[k] : 0u - stride[k];
-            }
-            active = cell[0] < g.res[0] && cell[0] > -1 && cell[1] < g.res[1] && cell[1] > -1 &&
-                     cell[2] < g.res[2] && cell[2] > -1;
-            c = (uint32_t)cell[0] + (uint32_t)cell[1] * stride[1] + (uint32_t)cell[2] * stride[2];
+        if (!clip(g, o, rcp, &t0, &t1)) return;
+        f3 ep = o;
+        if (t0 >= 0.0f) {
+            const float te = t0 + kEps;
+            ep = mk(o.x + te * d.x, o.y + te * d.y, o.z + te * d.z);
         }
+        const uint32_t stride[3] = {1u, (uint32_t)g.res[0], (uint32_t)g.res[0] * (uint32_t)g.res[1]};
+        bool inside = true;
+        cell = 0u;
+#pragma unroll
+        for (int k = 0; k < 3; ++k) {
+            float cf = floorf((comp(ep, k) - g.bmin[k]) * g.rcp[k]);
+            cf = hmin((float)g.res[k] - 1.0f, hmax(cf, 0.0f));
+            const bool fwd = rcp[k] > 0.0f;
+            const float stp = fwd ? 1.0f : 0.0f;
+            tmax[k] = ((cf + stp) * g.cs[k] + g.bmin[k] - comp(o, k)) * rcp[k];
+            dt[k] = g.cs[k] * fabsf(rcp[k]);
+            const int32_t c = f2i(cf);
+            inside = inside && c < g.res[k] && c > -1;
+            left[k] = fwd ? g.res[k] - 1 - c : c;
+            st3[k] = fwd ? stride[k] : 0u - stride[k];
+            cell += (uint32_t)c * stride[k];
+        }
+        st = inside ? 1 : 0;
     }
-    uint2 cr_next = make_uint2(0u, 0u);
-    bool have_next = false;
-    while (__any_sync(kFullMask, active)) {
-        uint32_t b = 0, e = 0;
-        if (active) {
-            const uint2 cr = have_next ? cr_next : __ldg(s.cells + c);
-            b = cr.x; e = cr.y;
+    __device__ __forceinline__ uint2 range(const Scene& s, Hit& h) const {
+        if (st == 0) return make_uint2(0u, 0u);
+        if (STATS) h.cells++;
+        return have_next ? cr_next : __ldg(s.cells + cell);
+    }
+    __device__ __forceinline__ void next(const Scene& s, const G& g, f3 o, f3 d, Hit& h, bool done) {
+        have_next = false;
+        if (st == 0) return;
+        if (done) {
+            st = 0;
+            return;
+        }
+        for (int j = 1;; ++j) {
+            float tk;
+            const bool inside = dda_step(tmax, dt, cell, st3, left, &tk);
+            if (!(h.t > tk && inside)) {
+                st = 0;
+                return;
+            }
+            if (j >= HR_UG_CELL_STEPS) return;
+            const uint2 nx = __ldg(s.cells + cell);
+            if (nx.y > nx.x) {
+                cr_next = nx;
+                have_next = true;
+                return;
+            }
             if (STATS) h.cells++;
         }
-        const bool done = test_lists<HM, STATS>(s, o, d, b, e, any, h);
-        have_next = false;
-        if (active) {
-            if (done) {
-                active = false;
-            } else {
-                for (int j = 1;; ++j) {
-                    float tk;
-                    const bool inside = dda_step(tmax, dt, c, st, left, &tk);
-                    active = h.t > tk && inside;
-                    if (!active || j >= HR_UG_CELL_STEPS) break;
-                    const uint2 nx = __ldg(s.cells + c);
-                    if (nx.y > nx.x) {
-                        cr_next = nx;
-                        have_next = true;
-                        break;
-                    }
-                    if (STATS) h.cells++;
-                }
-            }
-        }
     }
-}
+};
 
 // Two-level DDA state of one lane (TLGridTraverser.h:79-349).
 struct TL {
@@ -465,32 +474,16 @@ __device__ __forceinline__ bool tl_setup(TL& q, const Scene& s, const G& g, f3 o
     return tl_seek<STATS, OCC>(q, s, g, o, d, h);
 }
 
-// a15: two-level DDA, warp-synchronous
 #ifndef HR_RAY_LEAF_STEPS
-#define HR_RAY_LEAF_STEPS 4   // camera and query rays of trace_tl: leaves stepped per warp step while they are empty
+#define HR_RAY_LEAF_STEPS 4   // camera and query rays: leaves stepped per warp step while they are empty
 #endif
-template <int HM, bool STATS, bool OCC = false>
-__device__ void trace_tl(const Scene& s, const G& g, f3 o, f3 d, bool any, Hit& h, bool active) {
-    TL q;
-    if (active) active = tl_setup<STATS, OCC>(q, s, g, o, d, h);
-    while (__any_sync(kFullMask, active)) {
-        uint32_t b = 0, e = 0;
-        if (active) {
-            const uint2 lr = __ldg(s.leaves + q.leaf);
-            b = lr.x; e = lr.y;
-            if (STATS) h.cells++;
-        }
-        const bool done = test_lists<HM, STATS>(s, o, d, b, e, any, h);
-        if (active) active = !done && tl_advance<STATS, OCC, HR_RAY_LEAF_STEPS>(q, s, g, o, d, h);
-    }
-}
 
 // Paced two-level traversal, for path and shadow rays.  A lane walking empty top cells
 // takes at most K of them per warp step (and per call below), so one long walk does not
 // hold back the other lanes' leaf steps and list tests; each lane's own sequence of cells
 // and tests is unchanged, so the results are those of the unbounded walk.  Lane state: 0
-// done, 1 in a leaf, 2 walking empty top cells.  (Camera, AO and query rays keep the
-// unbounded walk of trace_tl: paced, they measured slower.)
+// done, 1 in a leaf, 2 walking empty top cells.  (Camera and AO rays keep the
+// unbounded walk: paced, they measured slower.)
 #ifndef HR_PT_SEEK_STEPS
 #define HR_PT_SEEK_STEPS 3   // path and shadow rays: empty top cells per warp step (0: unbounded)
 #endif
@@ -531,8 +524,9 @@ __device__ __forceinline__ int tl_setup_n(TL& q, const Scene& s, const G& g, f3 
 }
 
 // The lane state after a warp step: a lane in a leaf (st 1) whose list test ended the ray
-// (done) stops, else steps to the next leaf (tl_advance); a walking lane (st 2) walks on.
-template <bool STATS, bool OCC, int K>
+// (done) stops, else steps on over up to KL leaves while they are empty; a walking lane
+// (st 2) walks on.
+template <bool STATS, bool OCC, int K, int KL>
 __device__ __forceinline__ int tl_next(TL& q, const Scene& s, const G& g, f3 o, f3 d, Hit& h, int st, bool done) {
     if (st == 1) {
         if (done) return 0;
@@ -541,7 +535,7 @@ __device__ __forceinline__ int tl_next(TL& q, const Scene& s, const G& g, f3 o, 
             const bool inside = tl_leaf_step(q, &tk);
             if (h.t < tk) return 0;
             if (!inside) return tl_outer_step(q, h) ? tl_seek_n<STATS, OCC, K>(q, s, g, o, d, h) : 0;
-            if (j >= HR_PT_LEAF_STEPS) return 1;
+            if (j >= KL) return 1;
             // an empty leaf has no list to test: step over it within this warp step
             const uint2 lr = __ldg(s.leaves + q.leaf);
             if (lr.y > lr.x) return 1;
@@ -552,20 +546,110 @@ __device__ __forceinline__ int tl_next(TL& q, const Scene& s, const G& g, f3 o, 
     return 0;
 }
 
-// a15, paced (trace_tl's results)
-template <int HM, bool STATS, bool OCC, int K>
-__device__ void trace_tl_paced(const Scene& s, const G& g, f3 o, f3 d, bool any, Hit& h, bool active) {
+// a15: two-level DDA.  OCC: occupancy bits before cell records; SEEK: empty top cells
+// walked per warp step (0: all of them); KL: leaves stepped per warp step while empty.
+template <bool STATS, bool OCC, int SEEK, int KL>
+struct TravTL {
     TL q;
-    int st = active ? tl_setup_n<STATS, OCC, K>(q, s, g, o, d, h) : 0;
-    while (__any_sync(kFullMask, st != 0)) {
-        uint32_t b = 0, e = 0;
-        if (st == 1) {
-            const uint2 lr = __ldg(s.leaves + q.leaf);
-            b = lr.x; e = lr.y;
-            if (STATS) h.cells++;
+    int st;
+
+    __device__ __forceinline__ void start(const Scene& s, const G& g, f3 o, f3 d, Hit& h) {
+        if constexpr (SEEK > 0) st = tl_setup_n<STATS, OCC, SEEK>(q, s, g, o, d, h);
+        else st = tl_setup<STATS, OCC>(q, s, g, o, d, h) ? 1 : 0;
+    }
+    __device__ __forceinline__ uint2 range(const Scene& s, Hit& h) const {
+        if (st != 1) return make_uint2(0u, 0u);
+        if (STATS) h.cells++;
+        return __ldg(s.leaves + q.leaf);
+    }
+    __device__ __forceinline__ void next(const Scene& s, const G& g, f3 o, f3 d, Hit& h, bool done) {
+        if constexpr (SEEK > 0) st = tl_next<STATS, OCC, SEEK, KL>(q, s, g, o, d, h, st, done);
+        else if (st) st = !done && tl_advance<STATS, OCC, KL>(q, s, g, o, d, h) ? 1 : 0;
+    }
+};
+
+// the traverser of a grid kind for camera and query rays
+template <int KIND, bool STATS>
+using Trav = std::conditional_t<KIND == kUniform, TravUG<STATS>, TravTL<STATS, false, 0, HR_RAY_LEAF_STEPS>>;
+
+// One ray per lane until every lane's ray is done.  Warp-synchronous.
+template <class T, int HM, bool STATS>
+__device__ __forceinline__ void trace_lanes(const Scene& s, const G& g, f3 o, f3 d, bool any, Hit& h, bool active) {
+    T q;
+    q.st = 0;
+    if (active) q.start(s, g, o, d, h);
+    while (__any_sync(kFullMask, q.st != 0)) {
+        const uint2 r = q.range(s, h);
+        const bool done = test_lists<HM, STATS>(s, o, d, r.x, r.y, any, h);
+        q.next(s, g, o, d, h, done);
+    }
+}
+
+__device__ __forceinline__ void hit_reset(Hit& h, float tmax) {
+    h.t = tmax; h.u = 0.0f; h.v = 0.0f; h.tri = 0; h.hit = false; h.cells = 0; h.tests = 0;
+}
+
+// n rays shared out to the warps of a launch: at most `width` rays of a warp are in flight,
+// the first of them items warp * width ..., the others taken from the pool (next[0], which
+// counts from the first warps' items on; null when those are all) once `refill` of the
+// warp's lanes are idle.  next[0] and next[1] (warps that left) are zero between launches.
+struct RayPool {
+    uint32_t n, width, refill;
+    unsigned long long* next;
+};
+
+// Traces the rays of a pool: gen(item, o, d, h) sets up ray `item` (h.t its limit) and
+// returns whether there is one, fin(item, h, valid) takes its result.  A lane whose ray is
+// done waits until `refill` lanes of its warp (at most `width`) are; they then retire their
+// rays and take the next items together, so a warp keeps most of its lanes busy until the
+// pool is dry instead of stepping until its longest ray ends, and the set-up and the
+// result of a ray run for many lanes at once.
+template <class T, int HM, bool STATS, class Gen, class Fin>
+__device__ __forceinline__ void trace_pool(const Scene& s, const G& g, const RayPool& w, Gen gen, Fin fin) {
+    const uint32_t lane = threadIdx.x & 31u, lt = (1u << lane) - 1u;
+    const uint32_t wpb = blockDim.x >> 5, warps = gridDim.x * wpb;
+    const unsigned long long first = (unsigned long long)(blockIdx.x * wpb + (threadIdx.x >> 5)) * w.width;
+    T q;
+    q.st = 0;
+    Hit h;
+    hit_reset(h, FLT_MAX);
+    f3 o = mk(0.0f, 0.0f, 0.0f), d = mk(1.0f, 0.0f, 0.0f);
+    uint32_t item = 0;
+    bool has = false, valid = false, fresh = true, dry = false;
+    while (true) {
+        // lanes without a ray in flight: they retire theirs and take the next ones together
+        const uint32_t need = __ballot_sync(kFullMask, q.st == 0 && lane < w.width);
+        if ((uint32_t)__popc(need) >= w.refill) {   // warp-uniform
+            if (has && q.st == 0) fin(item, h, valid);
+            if (q.st == 0) has = false;
+            if (!dry) {
+                unsigned long long base = first;
+                if (!fresh) {
+                    if (lane == 0)
+                        base = (unsigned long long)warps * w.width + atomicAdd(w.next, (unsigned long long)__popc(need));
+                    base = __shfl_sync(kFullMask, base, 0);
+                }
+                fresh = false;
+                if (w.next == nullptr || base + (uint32_t)__popc(need) >= w.n) dry = true;
+                const unsigned long long i = base + __popc(need & lt);
+                if (((need >> lane) & 1u) && i < w.n) {
+                    item = (uint32_t)i;
+                    has = true;
+                    hit_reset(h, FLT_MAX);
+                    valid = gen(item, o, d, h);
+                    if (valid && s.ntri != 0u) q.start(s, g, o, d, h);
+                }
+            }
+            if (!__any_sync(kFullMask, has)) break;   // the pool is dry and no ray is in flight
         }
-        const bool done = test_lists<HM, STATS>(s, o, d, b, e, any, h);
-        st = tl_next<STATS, OCC, K>(q, s, g, o, d, h, st, done);
+        const uint2 r = q.range(s, h);
+        const bool done = test_lists<HM, STATS>(s, o, d, r.x, r.y, HM == kHitAny, h);
+        q.next(s, g, o, d, h, done);
+    }
+    // the last warp to leave clears the pool for the next launch
+    if (w.next && lane == 0 && atomicAdd(w.next + 1, 1ull) == warps - 1u) {
+        w.next[0] = 0ull;
+        w.next[1] = 0ull;
     }
 }
 
@@ -574,11 +658,10 @@ __device__ void trace_tl_paced(const Scene& s, const G& g, f3 o, f3 d, bool any,
 // registers of one traversal only.  Warp-synchronous.
 template <int KIND, bool ANY, bool STATS>
 __device__ __forceinline__ void trace_one(const Scene& s, const G& g, f3 o, f3 d, float tmax, Hit& h, bool active) {
-    h.t = tmax; h.u = 0.0f; h.v = 0.0f; h.tri = 0; h.hit = false; h.cells = 0; h.tests = 0;
+    hit_reset(h, tmax);
     if (s.ntri == 0) return;
     constexpr int HM = ANY ? kHitAny : kHitClosest;
-    if (KIND == kUniform) trace_ug<HM, STATS>(s, g, o, d, false, h, active);
-    else trace_tl<HM, STATS>(s, g, o, d, false, h, active);
+    trace_lanes<Trav<KIND, STATS>, HM, STATS>(s, g, o, d, false, h, active);
 }
 
 // As trace_one, with the hit mode chosen per lane: any hit where `any` is set, closest
@@ -587,12 +670,11 @@ __device__ __forceinline__ void trace_one(const Scene& s, const G& g, f3 o, f3 d
 template <int KIND, bool STATS, int SEEK = HR_PT_SEEK_STEPS>
 __device__ __forceinline__ void trace_mixed(const Scene& s, const G& g, f3 o, f3 d, float tmax, bool any, Hit& h,
                                             bool active) {
-    h.t = tmax; h.u = 0.0f; h.v = 0.0f; h.tri = 0; h.hit = false; h.cells = 0; h.tests = 0;
+    hit_reset(h, tmax);
     if (s.ntri == 0) return;
-    if (KIND == kUniform) trace_ug<kHitMixed, STATS>(s, g, o, d, any, h, active);
     // path rays: occupancy bits
-    else if constexpr (SEEK > 0) trace_tl_paced<kHitMixed, STATS, true, SEEK>(s, g, o, d, any, h, active);
-    else trace_tl<kHitMixed, STATS, true>(s, g, o, d, any, h, active);
+    using T = std::conditional_t<KIND == kUniform, TravUG<STATS>, TravTL<STATS, true, SEEK, HR_PT_LEAF_STEPS>>;
+    trace_lanes<T, kHitMixed, STATS>(s, g, o, d, any, h, active);
 }
 
 struct Cam {
@@ -927,18 +1009,20 @@ struct PathLane {
     bool has = false;
 };
 
-// Fill the lanes without a path from tile `tile` starting at slot *next (tile pixels as
-// tile_pixel); advances *next.  Returns the lanes still without a path.
-__device__ __forceinline__ uint32_t path_refill(PathLane& ln, const Cam& cam, uint32_t tile, uint32_t* next,
-                                               int32_t image_id, uint64_t seed, const float* __restrict__ fb) {
+// Fill the warp's first `width` lanes that have no path from the `width` pixel slots at
+// slot0 (slots as tile_pixel), starting at slot0 + *next; advances *next.  Returns the lanes
+// still without a path.
+__device__ __forceinline__ uint32_t path_refill(PathLane& ln, const Cam& cam, uint32_t slot0, uint32_t* next,
+                                               uint32_t width, int32_t image_id, uint64_t seed,
+                                               const float* __restrict__ fb) {
     const uint32_t lane = threadIdx.x & 31u;
-    uint32_t need = __ballot_sync(kFullMask, !ln.has);
-    while (need && *next < 32u) {
+    uint32_t need = __ballot_sync(kFullMask, !ln.has && lane < width);
+    while (need && *next < width) {
         const uint32_t rank = __popc(need & ((1u << lane) - 1u));
-        const uint32_t take = min((uint32_t)__popc(need), 32u - *next);
+        const uint32_t take = min((uint32_t)__popc(need), width - *next);
         if (!ln.has && rank < take) {
             uint32_t q;
-            if (tile_pixel(cam, tile * 32u + *next + rank, &q)) {
+            if (lane < width && tile_pixel(cam, slot0 + *next + rank, &q)) {
                 ln.pix = q;
                 ln.has = true;
                 ln.sample = 0;
@@ -947,7 +1031,7 @@ __device__ __forceinline__ uint32_t path_refill(PathLane& ln, const Cam& cam, ui
             }
         }
         *next += take;
-        need = __ballot_sync(kFullMask, !ln.has);
+        need = __ballot_sync(kFullMask, !ln.has && lane < width);
     }
     return need;
 }

@@ -76,3 +76,29 @@ def test_camera_rays_and_counters(engine, oracle, kind, res):
     for got, want in zip(out, (oid, ot, ou, ov)):
         assert np.array_equal(got.cpu().numpy(), want)
     assert np.array_equal(st.cpu().numpy().reshape(n, 2), np.asarray(ost).reshape(n, 2).astype(np.int32))
+
+
+@pytest.mark.parametrize("kind", [GRID_UNIFORM, GRID_TWO_LEVEL])
+def test_ray_queries_at_every_share_per_warp(engine, oracle, kind):
+    """Ray counts on both sides of each number of rays per warp, up to the refilled pool
+    (more rays than the resident warps hold), whose words the next query finds cleared."""
+    import torch
+    sms = torch.cuda.get_device_properties(0).multi_processor_count
+    full = sms * 32 * 32           # rays in flight at once: 32 warps per SM, 32 rays each
+    v, f = S.clusters(2000, seed=3)
+    b = build(engine, oracle, v, f, kind)
+    org, d = rays(full + 4097, 9)
+    oid, ot, ou, ov = oracle.trace(b, org, d)
+    tmax = np.full(len(org), 0.7, np.float32)
+    occ_o = np.asarray(oracle.occluded(b, org, d, tmax)).astype(bool)
+    do, dd, dt = (torch.from_numpy(x).cuda() for x in (org, d, tmax))
+    for n in (full // 32, full // 32 + 1, full // 8 + 5, full, full + 1, full + 4097, full + 4097, full // 2 + 1):
+        out = [torch.zeros(n, dtype=torch.int32, device="cuda")] + [torch.zeros(n, device="cuda") for _ in range(3)]
+        occ = torch.full((n,), 7, dtype=torch.uint8, device="cuda")
+        torch.cuda.synchronize()
+        engine.trace_rays_device(do, dd, n, *out)
+        engine.occluded_device(do, dd, dt, n, occ)
+        engine.sync()
+        for got, want in zip(out, (oid, ot, ou, ov)):
+            assert np.array_equal(got.cpu().numpy(), want[:n])
+        assert np.array_equal(occ.cpu().numpy().astype(bool), occ_o[:n])
