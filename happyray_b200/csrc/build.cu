@@ -135,7 +135,8 @@ template <bool EXACT>
 __global__ __launch_bounds__(kBT) void k_write_pairs(const float4* __restrict__ tris, uint32_t ntri, const GridDesc* d,
                                                      const uint32_t* block_sums, const uint4* __restrict__ rng,
                                                      uint32_t* __restrict__ keys, uint32_t* __restrict__ vals,
-                                                     uint32_t* __restrict__ cell_count) {
+                                                     uint32_t* __restrict__ cell_count, uint4* __restrict__ big,
+                                                     uint32_t* __restrict__ nbig) {
     if (d->overflow | d->error) return;
     const DescRegs g = load_desc(d);
     const uint32_t bx = gridDim.x - 1u - blockIdx.x;   // last block first (see k_leaf_write_pairs)
@@ -162,27 +163,50 @@ __global__ __launch_bounds__(kBT) void k_write_pairs(const float4* __restrict__ 
     }
     uint32_t tot;
     uint32_t slot = block_excl_scan<uint32_t, kBT>(n, &tot) + block_sums[bx];
-    if (n == 0) return;
-    const f3 nrm = normalize(cross(sub(p[1], p[0]), sub(p[2], p[0])));
-    const f3 h = mulf(g.cs, 0.505f);
-    f3 mc = mk((float)r.lo[0], (float)r.lo[1], (float)r.lo[2]);
-    mc = mk(mc.x * g.cs.x, mc.y * g.cs.y, mc.z * g.cs.z);
-    mc = add(add(mc, g.bmin), h);
-    f3 c;
-    c.z = mc.z - g.cs.z;
-    for (int32_t z = r.lo[2]; z < r.hi[2]; ++z) {
-        c.z += g.cs.z;
-        c.y = mc.y - g.cs.y;
-        for (int32_t y = r.lo[1]; y < r.hi[1]; ++y) {
-            c.y += g.cs.y;
-            c.x = mc.x - g.cs.x;
-            for (int32_t x = r.lo[0]; x < r.hi[0]; ++x, ++slot) {
-                c.x += g.cs.x;
-                keys[slot] = sat_overlap(nrm, c, p, h) ? (uint32_t)x + (uint32_t)y * rx + (uint32_t)z * rxy
-                                                       : g.ncells;
-                vals[slot] = t;
-            }
-        }
+    const bool written = exact_warp(
+        t, n, slot, g, [&](uint32_t tri, ExactTri& e) { tri_fetch(tris, tri, e.p); },
+        [&](uint32_t at, uint32_t key, uint32_t tri, bool) {
+            keys[at] = key;
+            vals[at] = tri;
+        });
+    if (n == 0 || written) return;
+    if (n > kExactWarp) {   // pieces for k_write_big_pairs (at most n / kExactWarp of them)
+        const uint32_t m = (n + kExactChunk - 1u) / kExactChunk, q = atomicAdd(nbig, m);
+        for (uint32_t i = 0; i < m; ++i) big[q + i] = make_uint4(t, slot, i * kExactChunk, min((i + 1u) * kExactChunk, n));
+        return;
+    }
+    ExactTri e;
+    e.p[0] = p[0]; e.p[1] = p[1]; e.p[2] = p[2];
+    e.r = r;
+    exact_tri(e, g);
+    exact_serial(e, g, [&](uint32_t key, bool) {
+        keys[slot] = key;
+        vals[slot] = t;
+        ++slot;
+    });
+}
+
+// a5, exact insertion of the triangles over many cells: a block per queued piece (triangle,
+// its first pair, cells [z, w) of its box).  Its threads also clear the cell ranges.
+__global__ __launch_bounds__(kBT) void k_write_big_pairs(const float4* __restrict__ tris, const GridDesc* d,
+                                                         const uint4* __restrict__ big, uint32_t* __restrict__ keys,
+                                                         uint32_t* __restrict__ vals, uint2* __restrict__ cells) {
+    if (d->overflow | d->error) return;
+    const DescRegs g = load_desc(d);
+    for (uint32_t c = blockIdx.x * kBT + threadIdx.x; c < g.ncells; c += gridDim.x * kBT) cells[c] = make_uint2(0u, 0u);
+    const uint32_t nbig = d->nbig;
+    for (uint32_t i = blockIdx.x; i < nbig; i += gridDim.x) {
+        const uint4 q = __ldg(big + i);
+        ExactTri e;
+        f3 lo, hi;
+        tri_fetch(tris, q.x, e.p);
+        tri_bbox(e.p, &lo, &hi);
+        cell_range(lo, hi, g.bmin, g.rcp, g.res, &e.r);
+        exact_tri(e, g);
+        exact_block<kBT, 1024>(e, g, q.z, q.w, [&](uint32_t l, uint32_t key, bool) {
+            keys[q.y + l] = key;
+            vals[q.y + l] = q.x;
+        });
     }
 }
 
@@ -309,7 +333,7 @@ static std::vector<uint8_t> build_graph_key(const hr_ctx* c, int32_t kind, int32
     const DevBuf* bufs[] = {&B.desc, &c->tris, &B.cells, &B.keys_a, &B.tri_ranges, &B.vals_a, &B.keys_b, &B.vals_b,
                             &B.block_sums, &B.tile_hist, &B.row_total, &B.prims,
                             &B.ref_ranges, &B.leaf_cnt, &B.occ, &B.scan_partials, &B.leaves, &B.lkeys_a, &B.lvals_a,
-                            &B.lkeys_b, &B.lvals_b, &c->verts, &c->idx, &c->counters, &c->keyframes, &c->frame_sel};
+                            &B.lkeys_b, &B.lvals_b, &B.big, &c->verts, &c->idx, &c->counters, &c->keyframes, &c->frame_sel};
     std::vector<uint8_t> k;
     auto put = [&](const void* p, size_t n) {
         const uint8_t* b = static_cast<const uint8_t*>(p);
@@ -386,6 +410,7 @@ static int build_once_impl(hr_ctx* c, int32_t kind, int32_t exact, uint32_t* ovf
         if ((rc = ensure(c, B.keys_b, sizeof(uint32_t) * cap_pairs))) return rc;
         if ((rc = ensure(c, B.vals_b, sizeof(uint32_t) * cap_pairs))) return rc;
         if ((rc = ensure(c, B.prims, sizeof(uint32_t) * cap_pairs))) return rc;
+        if (exact && (rc = ensure(c, B.big, sizeof(uint4) * (cap_pairs / kExactWarp + 1)))) return rc;
     } else {
         if ((rc = ensure(c, B.ref_ranges, sizeof(uint4) * cap_pairs))) return rc;
         if ((rc = ensure(c, B.leaf_cnt, sizeof(uint32_t) * B.cap_cells))) return rc;
@@ -429,12 +454,18 @@ static int build_once_impl(hr_ctx* c, int32_t kind, int32_t exact, uint32_t* ovf
             if ((rc = scan_block_sums(c, bsum, nblocks, d_np, &d->overflow, (uint32_t)std::min(cap_pairs, (size_t)0xffffffffu),
                                       kind == kUniform ? kOvfPairs : kOvfTopPairs, &d->req_pairs, s)))
                 return rc;
-            if (kind == kUniform && exact)
+            if (kind == kUniform && exact) {
                 k_write_pairs<true><<<nblocks, kBT, 0, s>>>(c->tris.as<float4>(), ntri, d, bsum, nullptr,
-                                                            B.keys_a.as<uint32_t>(), B.vals_a.as<uint32_t>(), nullptr);
-            else
+                                                            B.keys_a.as<uint32_t>(), B.vals_a.as<uint32_t>(), nullptr,
+                                                            B.big.as<uint4>(), &d->nbig);
+                k_write_big_pairs<<<c->num_sms * 8, kBT, 0, s>>>(c->tris.as<float4>(), d, B.big.as<uint4>(),
+                                                                 B.keys_a.as<uint32_t>(), B.vals_a.as<uint32_t>(),
+                                                                 B.cells.as<uint2>());
+            } else {
                 k_write_pairs<false><<<nblocks, kBT, 0, s>>>(c->tris.as<float4>(), ntri, d, bsum, B.tri_ranges.as<uint4>(),
-                                                             B.keys_a.as<uint32_t>(), B.vals_a.as<uint32_t>(), cell_count);
+                                                             B.keys_a.as<uint32_t>(), B.vals_a.as<uint32_t>(), cell_count,
+                                                             nullptr, nullptr);
+            }
         }
         mark();
         const int gcells = std::max(1, std::min((int)((B.cap_cells + 255) / 256), c->num_sms * 16));
@@ -447,7 +478,8 @@ static int build_once_impl(hr_ctx* c, int32_t kind, int32_t exact, uint32_t* ovf
                                        B.row_total.as<uint32_t>(), s)))
                 return rc;
             mark();
-            k_fill_u2<<<gcells, 256, 0, s>>>(B.cells.as<uint2>(), &d->ncells, d, make_uint2(0u, 0u));
+            if (!exact || nblocks == 0)   // k_write_big_pairs cleared them
+                k_fill_u2<<<gcells, 256, 0, s>>>(B.cells.as<uint2>(), &d->ncells, d, make_uint2(0u, 0u));
             const int gpairs = std::max(1, std::min((int)((cap_pairs + 255) / 256), c->num_sms * 16));
             k_cell_ranges<<<gpairs, 256, 0, s>>>(sorted_keys, d_np, &d->ncells, d, B.cells.as<uint2>());
             mark();

@@ -24,6 +24,7 @@ __device__ __forceinline__ void desc_init(GridDesc* d, int32_t kind, uint32_t nt
     d->ncells = d->npairs = d->ntop_pairs = d->nleaves = 0u;
     d->overflow = 0u;
     d->error = error;
+    d->nbig = 0u;
     d->kind = kind;
     d->ntri = ntri;
 }
@@ -125,6 +126,125 @@ __device__ __forceinline__ bool sat_overlap(f3 nrm, f3 c, const f3* tv, f3 h) {
     pass = pass && axis_test(-e2.z, e2.x, fe.z, fe.x, v0.x, v0.z, v1.x, v1.z, h.x, h.z);
     pass = pass && axis_test(e2.y, -e2.x, fe.y, fe.x, v1.x, v1.y, v2.x, v2.y, h.x, h.y);
     return pass;
+}
+
+// Exact insertion of one triangle over the cells of its bounding box (x, y, z order; a cell
+// the SAT test rejects gets key = ncells).  The cell centres are running sums along each
+// axis (UniformGridBuildKernels.cu:275-281), so a cell's centre depends on how it is
+// reached; formed in that order per axis, the cells can be tested in any order.  A triangle
+// of at most kExactSerial cells is written by its own thread, one of at most kExactWarp by
+// its warp, each lane walking the sums to its cells (unless so many of the warp's triangles
+// are alike that one thread each is quicker), and larger ones (a ground plane
+// spans tens of thousands of cells, which one thread walked in 5 ms on a 300k-triangle
+// scene) by blocks, kExactChunk cells at a time, from tables of the sums.
+constexpr uint32_t kExactSerial = 32u, kExactWarp = 512u, kExactChunk = 2048u;
+
+struct ExactTri {
+    f3 p[3], nrm, h, first;   // first: the centre sum before the first cell
+    CRange r;
+};
+__device__ __forceinline__ void exact_tri(ExactTri& e, const DescRegs& g) {
+    e.nrm = normalize(cross(sub(e.p[1], e.p[0]), sub(e.p[2], e.p[0])));
+    e.h = mulf(g.cs, 0.505f);
+    f3 mc = mk((float)e.r.lo[0], (float)e.r.lo[1], (float)e.r.lo[2]);
+    mc = mk(mc.x * g.cs.x, mc.y * g.cs.y, mc.z * g.cs.z);
+    mc = add(add(mc, g.bmin), e.h);
+    e.first = sub(mc, g.cs);
+}
+
+// the triangle's cells in order by one thread; put(key, inside) per cell
+template <class F>
+__device__ __forceinline__ void exact_serial(const ExactTri& e, const DescRegs& g, F put) {
+    const uint32_t rx = (uint32_t)g.res[0], rxy = (uint32_t)g.res[0] * (uint32_t)g.res[1];
+    f3 c;
+    c.z = e.first.z;
+    for (int32_t z = e.r.lo[2]; z < e.r.hi[2]; ++z) {
+        c.z += g.cs.z;
+        c.y = e.first.y;
+        for (int32_t y = e.r.lo[1]; y < e.r.hi[1]; ++y) {
+            c.y += g.cs.y;
+            c.x = e.first.x;
+            for (int32_t x = e.r.lo[0]; x < e.r.hi[0]; ++x) {
+                c.x += g.cs.x;
+                const bool in = sat_overlap(e.nrm, c, e.p, e.h);
+                put(in ? (uint32_t)x + (uint32_t)y * rx + (uint32_t)z * rxy : g.ncells, in);
+            }
+        }
+    }
+}
+
+// the triangles of a warp's lanes (triangle t of n cells, its first pair at slot) with
+// kExactSerial < n <= kExactWarp, one after another by all its lanes: fetch(t, e) loads a
+// triangle, put(at, key, t, inside) takes a cell's pair.  A warp with more of them than half
+// the cells of its largest leaves them to their threads (1000 triangles of a coarse
+// heightfield with a few over 17 to 27 cells per warp: build 0.059 ms, 0.070 with those by
+// the warp).  Returns
+// whether this lane's triangle was written; called by all lanes.
+template <class L, class F>
+__device__ __forceinline__ bool exact_warp(uint32_t t, uint32_t n, uint32_t slot, const DescRegs& g, L fetch, F put) {
+    const uint32_t lane = threadIdx.x & 31u;
+    const uint32_t rx = (uint32_t)g.res[0], rxy = (uint32_t)g.res[0] * (uint32_t)g.res[1];
+    const bool mine = n > kExactSerial && n <= kExactWarp;
+    const uint32_t all = __ballot_sync(0xffffffffu, mine);
+    if (all == 0u || 2u * (uint32_t)__popc(all) > __reduce_max_sync(0xffffffffu, mine ? n : 0u)) return false;
+    for (uint32_t m = all; m; m &= m - 1u) {
+        const int src = __ffs(m) - 1;
+        const uint32_t cells = __shfl_sync(0xffffffffu, n, src), tri = __shfl_sync(0xffffffffu, t, src);
+        const uint32_t at = __shfl_sync(0xffffffffu, slot, src);
+        ExactTri e;
+        f3 lo, hi;
+        fetch(tri, e);
+        tri_bbox(e.p, &lo, &hi);
+        cell_range(lo, hi, g.bmin, g.rcp, g.res, &e.r);
+        exact_tri(e, g);
+        const uint32_t ex = (uint32_t)(e.r.hi[0] - e.r.lo[0]), ey = (uint32_t)(e.r.hi[1] - e.r.lo[1]);
+        for (uint32_t l = lane; l < cells; l += 32u) {
+            const uint32_t a = l / ex, z = a / ey, x = l - a * ex, y = a - z * ey;
+            f3 c = e.first;
+            for (uint32_t i = 0; i <= x; ++i) c.x += g.cs.x;
+            for (uint32_t i = 0; i <= y; ++i) c.y += g.cs.y;
+            for (uint32_t i = 0; i <= z; ++i) c.z += g.cs.z;
+            const bool in = sat_overlap(e.nrm, c, e.p, e.h);
+            const uint32_t key = (uint32_t)e.r.lo[0] + x + ((uint32_t)e.r.lo[1] + y) * rx + ((uint32_t)e.r.lo[2] + z) * rxy;
+            put(at + l, in ? key : g.ncells, tri, in);
+        }
+    }
+    return mine;
+}
+
+// cells [l0, l1) of the triangle's box by a block of NT threads; put(l, key, inside) per
+// cell.  The first TAB cells of an axis have table entries, beyond them a thread walks the
+// sum.  Every thread of the block calls it with the same arguments.
+template <int NT, int TAB, class F>
+__device__ __forceinline__ void exact_block(const ExactTri& e, const DescRegs& g, uint32_t l0, uint32_t l1, F put) {
+    __shared__ float s_c[3][TAB];
+    const uint32_t rx = (uint32_t)g.res[0], rxy = (uint32_t)g.res[0] * (uint32_t)g.res[1];
+    const uint32_t ex = (uint32_t)(e.r.hi[0] - e.r.lo[0]), ey = (uint32_t)(e.r.hi[1] - e.r.lo[1]);
+    __syncthreads();   // the table of the previous call
+    if (threadIdx.x < 3) {
+        const int k = (int)threadIdx.x;
+        const int n = min(e.r.hi[k] - e.r.lo[k], TAB);
+        const float cs = comp(g.cs, k);
+        float v = comp(e.first, k);
+        for (int i = 0; i < n; ++i) {
+            v += cs;
+            s_c[k][i] = v;
+        }
+    }
+    __syncthreads();
+    for (uint32_t l = l0 + threadIdx.x; l < l1; l += NT) {
+        const uint32_t a = l / ex, z = a / ey;
+        const uint32_t q[3] = {l - a * ex, a - z * ey, z};
+        float cc[3];
+#pragma unroll
+        for (int k = 0; k < 3; ++k) {
+            cc[k] = s_c[k][min(q[k], (uint32_t)TAB - 1u)];
+            for (uint32_t i = TAB; i <= q[k]; ++i) cc[k] += comp(g.cs, k);
+        }
+        const bool in = sat_overlap(e.nrm, mk(cc[0], cc[1], cc[2]), e.p, e.h);
+        const uint32_t x = (uint32_t)e.r.lo[0] + q[0], y = (uint32_t)e.r.lo[1] + q[1], zz = (uint32_t)e.r.lo[2] + q[2];
+        put(l, in ? x + y * rx + zz * rxy : g.ncells, in);
+    }
 }
 
 __global__ void k_fill_u2(uint2* a, const uint32_t* d_count, const GridDesc* d, uint2 val) {

@@ -9,7 +9,8 @@
 //   1  key-frame lerp + per-block bounds                            (k_lerp_bounds)
 //   2  bounds of all blocks, resolution; per-triangle pair count    (k_grid_setup, k_count_pairs)
 //   3  scan of the block counts, pair scatter (k_scan_block_sums, k_write_pairs); each
-//      accepted pair also counted in its cell
+//      accepted pair also counted in its cell; with exact insertion, triangles over many
+//      cells are shared out to all blocks after one more barrier (k_write_big_pairs)
 //   4  per block: a chunk of cells (pair sum, longest list), a chunk of pairs (rejected)
 //   5  cell starts by scan of the counts: cells[c] = (start, start), (0, 0) if empty
 //   6  placement: an accepted pair at its cell's cursor (cells[c].y, an atomic add that
@@ -41,6 +42,7 @@ static_assert(kBT == kThreads, "the build block is the radix block");
 
 constexpr uint32_t kBarrierPolls = 1u << 21;   // under a second of polling (one L2 round trip each)
 constexpr uint32_t kCountListMax = 32;          // longest cell list placed by counting
+constexpr uint32_t kSmallPiece = kBT;           // cells of a large triangle that a block takes at once
 constexpr int kRun = 8;                         // a thread's cells whose counts stay in registers
 
 struct SmallUG {
@@ -62,6 +64,7 @@ struct SmallUG {
     uint32_t* bar;               // {arrivals, generation}
     int32_t* blk_bounds;         // 6 encoded bounds per block
     uint32_t* blk_pairs;         // pair count per block
+    uint32_t* blk_piece;         // pieces of its triangles over many cells
     uint32_t *blk_csum, *blk_cmax, *blk_rej;   // per block: its cells' pairs, longest list, rejected pairs
 };
 
@@ -163,7 +166,7 @@ __device__ __forceinline__ uint64_t block_sum_u64(uint64_t x) {
     return t;
 }
 
-__global__ __launch_bounds__(kBT) void k_build_ug_small(SmallUG P) {
+__global__ __launch_bounds__(kBT, 3) void k_build_ug_small(SmallUG P) {
     __shared__ GridDesc s_d;
     __shared__ int32_t s_enc[6];
     const uint32_t G = gridDim.x, b = blockIdx.x, tid = threadIdx.x;
@@ -283,9 +286,15 @@ __global__ __launch_bounds__(kBT) void k_build_ug_small(SmallUG P) {
         tri_bbox(p, &lo, &hi);
         n = cell_range(lo, hi, g.bmin, g.rcp, g.res, &r);
     }
-    uint32_t btot;
-    const uint32_t ex = block_excl_scan<uint32_t, kBT>(n, &btot);
-    if (tid == 0) P.blk_pairs[b] = btot;
+    // with exact insertion also the pieces of triangles over many cells
+    uint2 btot;
+    const uint32_t npiece = P.exact && n > kExactWarp ? (n + kSmallPiece - 1u) / kSmallPiece : 0u;
+    const uint2 ex2 = block_excl_scan<uint2, kBT>(make_uint2(n, npiece), &btot);
+    const uint32_t ex = ex2.x;
+    if (tid == 0) {
+        P.blk_pairs[b] = btot.x;
+        P.blk_piece[b] = btot.y;
+    }
     // the cells' .y words count the accepted pairs of each cell in phase 3
     for (uint32_t c = b * kBT + tid; c < g.ncells; c += G * kBT) P.cells[c] = make_uint2(0u, 0u);
     if (!grid_barrier(P.bar, P.d)) return;
@@ -294,12 +303,17 @@ __global__ __launch_bounds__(kBT) void k_build_ug_small(SmallUG P) {
     // pairs go to their slots as k_write_pairs writes them, and every accepted pair is
     // counted in its cell
     uint64_t mine = 0, all = 0;
+    uint32_t pmine = 0, pall = 0;
     for (uint32_t j = tid; j < G; j += kBT) {
-        const uint32_t x = __ldcg(P.blk_pairs + j);
+        const uint32_t x = __ldcg(P.blk_pairs + j), y = __ldcg(P.blk_piece + j);
         all += x;
-        if (j < b) mine += x;
+        pall += y;
+        if (j < b) { mine += x; pmine += y; }
     }
     const uint64_t pre64 = block_sum_u64(mine), total = block_sum_u64(all);
+    // pieces before this block's in the high half, all of them in the low half (each below
+    // 2^32 / kExactWarp)
+    const uint64_t pieces = P.exact ? block_sum_u64((uint64_t)pmine << 32 | pall) : 0ull;
     if (total > (uint64_t)P.cap_pairs) {
         if (b == 0 && tid == 0) {
             atomicOr(&P.d->overflow, kOvfPairs);
@@ -315,30 +329,44 @@ __global__ __launch_bounds__(kBT) void k_build_ug_small(SmallUG P) {
     if (P.exact) {
         // each triangle's bounding-box cells in x, y, z order; a cell the SAT test rejects
         // gets key = ncells (sorted last, skipped by the ranges)
-        if (n) {
-            uint32_t slot = pre + ex;
-            const f3 nrm = normalize(cross(sub(p[1], p[0]), sub(p[2], p[0])));
-            const f3 h = mulf(g.cs, 0.505f);
-            f3 mc = mk((float)r.lo[0], (float)r.lo[1], (float)r.lo[2]);
-            mc = mk(mc.x * g.cs.x, mc.y * g.cs.y, mc.z * g.cs.z);
-            mc = add(add(mc, g.bmin), h);
-            f3 c;
-            c.z = mc.z - g.cs.z;
-            for (int32_t z = r.lo[2]; z < r.hi[2]; ++z) {
-                c.z += g.cs.z;
-                c.y = mc.y - g.cs.y;
-                for (int32_t y = r.lo[1]; y < r.hi[1]; ++y) {
-                    c.y += g.cs.y;
-                    c.x = mc.x - g.cs.x;
-                    for (int32_t x = r.lo[0]; x < r.hi[0]; ++x, ++slot) {
-                        c.x += g.cs.x;
-                        const bool in = sat_overlap(nrm, c, p, h);
-                        const uint32_t key = in ? (uint32_t)x + (uint32_t)y * rx + (uint32_t)z * rxy : C;
-                        P.keys_a[slot] = key;
-                        P.vals_a[slot] = t;
-                        if (in) atomicAdd(cnt + 2 * (size_t)key, 1u);
-                    }
-                }
+        const uint32_t slot0 = pre + ex;
+        auto fetch = [&](uint32_t tri, ExactTri& e) {   // written by this launch
+            const float4* q = P.tris + 3 * (size_t)tri;
+            const float4 q0 = __ldcg(q), q1 = __ldcg(q + 1), q2 = __ldcg(q + 2);
+            e.p[0] = mk(q0.x, q0.y, q0.z); e.p[1] = mk(q1.x, q1.y, q1.z); e.p[2] = mk(q2.x, q2.y, q2.z);
+        };
+        auto put = [&](uint32_t at, uint32_t key, uint32_t tri, bool in) {
+            P.keys_a[at] = key;
+            P.vals_a[at] = tri;
+            if (in) atomicAdd(cnt + 2 * (size_t)key, 1u);
+        };
+        const bool written = exact_warp(t, n, slot0, g, fetch, put);
+        if (n && n <= kExactWarp && !written) {
+            ExactTri e;
+            e.p[0] = p[0]; e.p[1] = p[1]; e.p[2] = p[2];
+            e.r = r;
+            exact_tri(e, g);
+            uint32_t slot = slot0;
+            exact_serial(e, g, [&](uint32_t key, bool in) { put(slot++, key, t, in); });
+        }
+        // triangles over many cells: their pieces (triangle, first pair, cells) go to a list
+        // (the sort's buffer, not in use yet), which all blocks then share
+        const uint32_t npieces = (uint32_t)pieces;
+        if (npieces) {
+            uint4* const list = reinterpret_cast<uint4*>(P.keys_b);
+            for (uint32_t i = 0; i < npiece; ++i)
+                list[(uint32_t)(pieces >> 32) + ex2.y + i] =
+                    make_uint4(t, slot0, i * kSmallPiece, min((i + 1u) * kSmallPiece, n));
+            if (!grid_barrier(P.bar, P.d)) return;
+            for (uint32_t i = b; i < npieces; i += G) {
+                const uint4 q = __ldcg(list + i);
+                ExactTri e;
+                f3 lo, hi;
+                fetch(q.x, e);
+                tri_bbox(e.p, &lo, &hi);
+                cell_range(lo, hi, g.bmin, g.rcp, g.res, &e.r);
+                exact_tri(e, g);
+                exact_block<kBT, 96>(e, g, q.z, q.w, [&](uint32_t l, uint32_t key, bool in) { put(q.y + l, key, q.x, in); });
             }
         }
     } else {
@@ -514,7 +542,7 @@ int build_small_uniform(hr_ctx* c, int32_t exact, int key_bits, bool* done) {
     // streams always fit side by side
     const uint32_t G = std::max((ntri + kBT - 1) / kBT, (uint32_t)c->num_sms);
     if (c->small_build_bps <= 0 || 2 * G > (uint32_t)c->small_build_bps * (uint32_t)c->num_sms) return 0;
-    const size_t bar_words = 4, bytes = sizeof(uint32_t) * (bar_words + 10 * (size_t)G);
+    const size_t bar_words = 4, bytes = sizeof(uint32_t) * (bar_words + 11 * (size_t)G);
     const void* before = c->build_bar.p;
     const size_t before_bytes = c->build_bar.bytes;
     int rc;
@@ -557,6 +585,7 @@ int build_small_uniform(hr_ctx* c, int32_t exact, int key_bits, bool* done) {
     P.blk_csum = P.blk_pairs + G;
     P.blk_cmax = P.blk_csum + G;
     P.blk_rej = P.blk_cmax + G;
+    P.blk_piece = P.blk_rej + G;
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3(G);
     cfg.blockDim = dim3(kBT);

@@ -261,7 +261,7 @@ void hr_destroy(hr_ctx* c) {
                       &c->g.prims, &c->g.keys_a, &c->g.vals_a, &c->g.keys_b, &c->g.vals_b, &c->g.block_sums,
                       &c->g.tile_hist, &c->g.row_total, &c->g.leaf_cnt, &c->g.occ,
                       &c->g.lkeys_a, &c->g.lvals_a, &c->g.lkeys_b, &c->g.lvals_b, &c->g.scan_partials,
-                      &c->g.tri_ranges, &c->g.ref_ranges, &c->lights_dev, &c->tri_nrm, &c->tri_alb,
+                      &c->g.tri_ranges, &c->g.big, &c->g.ref_ranges, &c->lights_dev, &c->tri_nrm, &c->tri_alb,
                       &c->hit_t, &c->hit_tri, &c->unocc, &c->queue, &c->build_bar};
     for (DevBuf* b : bufs) free_buf(c, *b);
     cudaStreamSynchronize(c->stream);

@@ -47,7 +47,7 @@ struct GridDesc {
     uint32_t req_cells;   // cells needed when kOvfCells is set (ncells is then 0)
     uint32_t req_pairs;   // pairs needed when kOvfPairs / kOvfTopPairs is set (count is then 0)
     uint32_t req_leaf_pairs;   // leaf pairs needed when kOvfLeafPairs is set (count is then 0)
-    uint32_t pad1;
+    uint32_t nbig;        // exact uniform build: pieces of large triangles queued by k_write_pairs
 };
 
 // Area lights of the path tracer (AreaLightSource, LightSource.hpp:38-95): parallelogram
