@@ -295,9 +295,10 @@ __global__ __launch_bounds__(kTT, HR_TRACE_MIN_BLOCKS) void k_ao_samples(Scene s
     const f3 cpos = mk(cam.pos[0], cam.pos[1], cam.pos[2]);
     const uint32_t nitems = *qcount * (uint32_t)spp;
     const uint32_t lane = threadIdx.x & 31u, lt = (1u << lane) - 1u;
-    // rays a warp holds at a time (as ray_width): fewer where the items would not fill the warps
+    // rays a warp holds at a time (as ray_width): fewer where the items would not fill the warps,
+    // at least 8
     uint32_t width = 32u;
-    while (width > 1u && nitems < gridDim.x * (kTT / 32u) * width) width /= 2u;
+    while (width > 8u && nitems < gridDim.x * (kTT / 32u) * width) width /= 2u;
     AoTrav<KIND, STATS> q;
     q.st = 0;
     Hit h;
@@ -453,21 +454,29 @@ Cam make_cam(const hr_ctx* c) {
 // a smaller power of two (at least `least`) while n rays would not fill them `waves` times.
 // A warp step costs the longest of its lanes' walks, and a small launch is as long as its
 // slowest warp: with fewer rays per warp the walks are shorter, a ray's list is still
-// tested by all 32 lanes, and the GPU's other warps take the rest.
+// tested by all 32 lanes, and the GPU's other warps take the rest; the launch as a whole
+// does more work.
 uint32_t ray_width(uint64_t n, uint64_t warps, uint32_t waves, uint32_t least) {
     uint32_t w = 32u;
     while (w > least && n < warps * w * waves) w /= 2u;
     return w;
 }
 
-// Camera rays: warps filled four times over, at least 4 rays each (coherent rays share their
-// walk, and the short launches' tail is a tile over dense cells).  Per ms at 32 / 16 / 8 / 4
-// rays: 256 x 256 uniform heightfield 0.067 / 0.061 / 0.054 / 0.051, 640 x 480 two-level
-// 100k 0.157 / 0.149 / 0.166 / 0.227, 801 x 601 uniform grid with lists of thousands 2.56 /
-// 1.45 / 1.34 / 1.68, 1080p two-level 1M 0.586 / 0.779 / 1.29 / 2.14.
-uint32_t camera_width(const hr_ctx* c) {
+// Camera rays.  Coherent rays share their walk, so a narrower warp saves less of a step than
+// it gives up, and next to other work on the GPU the work counts, not the launch's tail.
+// Two-level grids: 32 rays unless the image does not fill a quarter of the warps, at least 8
+// (a frame, passes overlapping / alone, at 32 / 16 / 8 / 4 rays: 128 x 128 113 / 86 / 87 / 92 us
+// and 194 / 198 / 167 / 141, 313 x 308 160 / 165 / 183 / 209 and 294 / 275 / 263 / 276).
+// Uniform grids, whose crowded cells make tiles of very uneven cost: warps filled four
+// times over, at least 4 rays (256 x 256 97 us at 32, 87 at 4; 801 x 601 with lists of
+// thousands 883 at 32, 679 at 16; kernels alone 0.067 -> 0.051 and 2.56 -> 1.45 ms).  AO
+// camera rays on two-level grids: four times over, at least 16 (641 x 479, where 32-ray
+// tiles are just over two per warp: 0.212 -> 0.155 ms).
+uint32_t camera_width(const hr_ctx* c, bool ao) {
     const uint64_t slots = (((uint64_t)c->cam.w + 7u) / 8u) * (((uint64_t)c->cam.h + 3u) / 4u) * 32u;
-    return ray_width(slots, (uint64_t)c->num_sms * HR_TRACE_MIN_BLOCKS * (kTT / 32), 4, 4);
+    const uint64_t warps = (uint64_t)c->num_sms * HR_TRACE_MIN_BLOCKS * (kTT / 32);
+    if (c->built_kind == kUniform) return ray_width(slots, warps, 4, 4);
+    return ao ? ray_width(slots, warps, 4, 16) : ray_width(slots, warps / 4u, 1, 8);
 }
 
 // The pool of a ray query over n rays and its block count (blocks resident at once; the
@@ -532,7 +541,7 @@ int launch_trace_primary(hr_ctx* c, int32_t* id, float* t, float* u, float* v, u
     const uint32_t n = (uint32_t)k.w * (uint32_t)k.h;
     if (n == 0) return 0;
     c->launches += 1;
-    const uint32_t width = camera_width(c);
+    const uint32_t width = camera_width(c, false);
     by_kind(s.kind, stats != nullptr, [&](auto K, auto S) {
         k_trace_primary<K(), S()><<<grid_for(c, slots_for(c) / width * 32u), kTT, 0, c->stream>>>(s, k, width, id, t, u, v,
                                                                                                  stats);
@@ -577,7 +586,7 @@ int launch_render(hr_ctx* c, int32_t mode, int32_t image_id, float* d_fb) {
     c->nrender_ev = 0;
     switch (mode) {
     case 0: {
-        const uint32_t width = camera_width(c);
+        const uint32_t width = camera_width(c, false);
         const int gw = grid_for(c, slots_for(c) / width * 32u);
         c->launches += 1;
         mark(0);
@@ -600,7 +609,8 @@ int launch_render(hr_ctx* c, int32_t mode, int32_t image_id, float* d_fb) {
                 cudaGetLastError();
                 nb = 1;
             }
-            const uint32_t width = ray_width(slots_for(c), (uint64_t)nb * c->num_sms * (kTT / 32), 1, 1);
+            // 320 x 200 at 32 / 16 / 8 / 4 paths per warp: 718 / 596 / 532 / 539 us a four-image pass
+            const uint32_t width = ray_width(slots_for(c), (uint64_t)nb * c->num_sms * (kTT / 32), 1, 8);
             const uint32_t need = (slots_for(c) / width + kTT / 32 - 1) / (kTT / 32);   // blocks
             const int gp = (int)std::min(need, (uint32_t)(nb * c->num_sms));
             k_render_pt<K(), S()><<<gp, kTT, 0, strm>>>(s, k, l, c->ip.pt_bounces, c->ip.albedo, c->ip.ray_eps_frac,
@@ -623,7 +633,7 @@ int launch_render(hr_ctx* c, int32_t mode, int32_t image_id, float* d_fb) {
         mark(0);
         // blocks of both kernels: all resident at once (the launch bounds allow HR_TRACE_MIN_BLOCKS per SM)
         const int nb = HR_TRACE_MIN_BLOCKS * c->num_sms;
-        const uint32_t width = camera_width(c);
+        const uint32_t width = camera_width(c, true);
         by_kind(s.kind, st, [&](auto K, auto S) {
             k_ao_primary<K(), S()><<<std::min(grid_for(c, slots_for(c) / width * 32u), nb), kTT, 0, strm>>>(
                 s, k, image_id, d_fb, c->hit_t.as<float>(), c->hit_tri.as<uint32_t>(), c->unocc.as<uint32_t>(),
