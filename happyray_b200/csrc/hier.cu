@@ -28,10 +28,7 @@
 #include <vector>
 
 #ifndef HR_HIER_MIN_BLOCKS
-#define HR_HIER_MIN_BLOCKS 8   // blocks per SM the trace kernel's register budget must allow (8: 64 registers)
-#endif
-#ifndef HR_HIER_WARP_POOL
-#define HR_HIER_WARP_POOL 1   // trace warps take 32 consecutive rays from a pool once all lanes are done
+#define HR_HIER_MIN_BLOCKS 6   // blocks per SM the trace kernel's register budget must allow (6: 80 registers)
 #endif
 
 namespace hr {
@@ -220,24 +217,36 @@ __global__ __launch_bounds__(kBT) void k_hier_write(const float4* __restrict__ t
 // One block: the union of the instance boxes, padded as the scene bounds
 // (WFObjectUploader.h:112-114); resolution max(1, (int)(diag * (density * n /
 // volume)^(1/3))) (TLGridHierarchySortBuilder.cu:275-286), cell size diag / res
-// (TLGridHierarchyMemoryManager.h:111-119).
-__global__ __launch_bounds__(kBT) void k_hier_top_setup(const HierInst* __restrict__ inst, uint32_t ninst,
-                                                        float density, GridDesc* __restrict__ d) {
+// (TLGridHierarchyMemoryManager.h:111-119).  1024 threads with four boxes in flight each and
+// a shuffle reduction: 16,384 boxes 30 -> 8 us (256 threads, the last step one thread's).
+constexpr int kTopThreads = 1024;
+__global__ __launch_bounds__(kTopThreads) void k_hier_top_setup(const HierInst* __restrict__ inst, uint32_t ninst,
+                                                                float density, GridDesc* __restrict__ d) {
     f3 lo = mk(FLT_MAX, FLT_MAX, FLT_MAX), hi = mk(-FLT_MAX, -FLT_MAX, -FLT_MAX);
-    for (uint32_t i = threadIdx.x; i < ninst; i += kBT) {
-        const float4 a = inst[i].lo, b = inst[i].hi;
+#pragma unroll 4
+    for (uint32_t i = threadIdx.x; i < ninst; i += kTopThreads) {
+        const float4 a = __ldg(&inst[i].lo), b = __ldg(&inst[i].hi);
         lo = vmin(lo, mk(a.x, a.y, a.z));
         hi = vmax(hi, mk(b.x, b.y, b.z));
     }
-    __shared__ float s[6][kBT];
-    s[0][threadIdx.x] = lo.x; s[1][threadIdx.x] = lo.y; s[2][threadIdx.x] = lo.z;
-    s[3][threadIdx.x] = hi.x; s[4][threadIdx.x] = hi.y; s[5][threadIdx.x] = hi.z;
+    __shared__ f3 s_lo[kTopThreads / 32], s_hi[kTopThreads / 32];
+    auto reduce = [&]() {
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) {
+            lo = vmin(lo, mk(__shfl_xor_sync(kFullMask, lo.x, o), __shfl_xor_sync(kFullMask, lo.y, o),
+                             __shfl_xor_sync(kFullMask, lo.z, o)));
+            hi = vmax(hi, mk(__shfl_xor_sync(kFullMask, hi.x, o), __shfl_xor_sync(kFullMask, hi.y, o),
+                             __shfl_xor_sync(kFullMask, hi.z, o)));
+        }
+    };
+    reduce();
+    if ((threadIdx.x & 31u) == 0u) { s_lo[threadIdx.x >> 5] = lo; s_hi[threadIdx.x >> 5] = hi; }
     __syncthreads();
-    if (threadIdx.x != 0) return;
-    for (int j = 1; j < kBT; ++j) {
-        lo = vmin(lo, mk(s[0][j], s[1][j], s[2][j]));
-        hi = vmax(hi, mk(s[3][j], s[4][j], s[5][j]));
-    }
+    if (threadIdx.x >= 32u) return;
+    lo = s_lo[threadIdx.x];
+    hi = s_hi[threadIdx.x];
+    reduce();
+    if (threadIdx.x != 0u) return;
     const f3 dd = sub(hi, lo);
     const float pad = 0.001f * sqrtf(dot(dd, dd));
     d->bmin[0] = lo.x - pad; d->bmin[1] = lo.y - pad; d->bmin[2] = lo.z - pad;
@@ -333,155 +342,76 @@ __device__ __forceinline__ void box_clip(const float* bmin, const float* bmax, f
     *t1 = hmin(hmin(tf[0], tf[1]), tf[2]);
 }
 
-struct HHit {
-    float t, u, v;
-    int32_t inst, tri;
-};
-
 // per-ray work counters (STATS instances): instance-grid cells, instance boxes tested,
 // instances entered, object-grid cells, triangle tests
 struct HCount {
     uint32_t top_cells = 0, inst_tests = 0, inst_entered = 0, obj_cells = 0, tri_tests = 0;
 };
 
-// One instance (GeometryInstanceTraverser, TLGridHierarchyTraverser.h:45-205): the world
-// box interval, the ray in object space, the object grid's DDA from the current best t.
-// Returns true when the instance's hit is accepted (inside the box interval, closer).
-template <bool STATS>
-__device__ bool hier_instance(const HierView& H, uint32_t ii, f3 o, f3 d, const float* rcp, HHit& h, HCount& n) {
-    const HierInst I = H.inst[ii];
-    const float blo[3] = {I.lo.x, I.lo.y, I.lo.z}, bhi[3] = {I.hi.x, I.hi.y, I.hi.z};
-    float te1, tx1;
-    box_clip(blo, bhi, o, rcp, &te1, &tx1);
-    if (STATS) n.inst_tests++;
-    if (!(tx1 > te1 && tx1 >= 0.0f && te1 < h.t)) return false;
-    if (STATS) n.inst_entered++;
-    const f3 ot = mk(I.r0.x * o.x + I.r0.y * o.y + I.r0.z * o.z + I.r0.w,
-                     I.r1.x * o.x + I.r1.y * o.y + I.r1.z * o.z + I.r1.w,
-                     I.r2.x * o.x + I.r2.y * o.y + I.r2.z * o.z + I.r2.w);
-    const f3 dt = mk(I.r0.x * d.x + I.r0.y * d.y + I.r0.z * d.z, I.r1.x * d.x + I.r1.y * d.y + I.r1.z * d.z,
-                     I.r2.x * d.x + I.r2.y * d.y + I.r2.z * d.z);
-    const float rt[3] = {1.0f / dt.x, 1.0f / dt.y, 1.0f / dt.z};
-    const HierObj g = H.objs[__float_as_uint(I.lo.w)];
-    Scene s;
-    s.tris = H.tris;
-    float rayT = h.t, bu = 0.0f, bv = 0.0f;
-    int32_t best = -1;
-    float te, tx;
-    box_clip(g.bmin, g.bmax, ot, rt, &te, &tx);
-    bool flag = tx > te && tx >= 0.0f && te < rayT;
-    f3 ep = ot;
-    if (te >= 0.0f) {
-        const float sc = te + kEps;
-        ep = mk(ot.x + sc * dt.x, ot.y + sc * dt.y, ot.z + sc * dt.z);
-    }
-    float tmax[3];
-    int32_t cell[3];
-#pragma unroll
-    for (int k = 0; k < 3; ++k) {
-        float cf = floorf((comp(ep, k) - g.bmin[k]) * g.rcp[k]);
-        cf = rt[k] > 0.0f ? hmin((float)g.res[k] - 1.0f, cf) : hmax(cf, 0.0f);
-        const float stp = rt[k] > 0.0f ? 1.0f : 0.0f;
-        tmax[k] = ((cf + stp) * g.cs[k] + g.bmin[k] - comp(ot, k)) * rt[k];
-        cell[k] = f2i(cf);
-        flag = flag && (rt[k] > 0.0f ? cell[k] < g.res[k] : cell[k] > -1);
-    }
-    const uint32_t rx = (uint32_t)g.res[0], rxy = (uint32_t)g.res[0] * (uint32_t)g.res[1];
-    while (flag) {
-        if (cell[0] < g.res[0] && cell[0] > -1 && cell[1] < g.res[1] && cell[1] > -1 && cell[2] < g.res[2] &&
-            cell[2] > -1) {
-            const uint2 cr = __ldg(H.obj_cells + (g.cell_off + (uint32_t)cell[0] + (uint32_t)cell[1] * rx +
-                                                  (uint32_t)cell[2] * rxy));
-            if (STATS) {
-                n.obj_cells++;
-                n.tri_tests += cr.y - cr.x;
-            }
-            for (uint32_t it = cr.x; it < cr.y; ++it) {
-                const uint32_t tri = __ldg(H.prims + it);
-                float t, u, v;
-                if (mt_test(s, tri, ot, dt, rayT, &t, &u, &v)) {
-                    rayT = t; bu = u; bv = v; best = (int32_t)tri;
-                }
-            }
-        }
-        const int k = min_dim(tmax[0], tmax[1], tmax[2]);
-        float tk;
-        if (k == 0) {
-            tk = tmax[0];
-            cell[0] += rt[0] > 0.0f ? 1 : -1;
-            tmax[0] += g.cs[0] * fabsf(rt[0]);
-            flag = flag && rayT > tk && (rt[0] > 0.0f ? cell[0] < g.res[0] : cell[0] > -1);
-        } else if (k == 1) {
-            tk = tmax[1];
-            cell[1] += rt[1] > 0.0f ? 1 : -1;
-            tmax[1] += g.cs[1] * fabsf(rt[1]);
-            flag = flag && rayT > tk && (rt[1] > 0.0f ? cell[1] < g.res[1] : cell[1] > -1);
-        } else {
-            tk = tmax[2];
-            cell[2] += rt[2] > 0.0f ? 1 : -1;
-            tmax[2] += g.cs[2] * fabsf(rt[2]);
-            flag = flag && rayT > tk && (rt[2] > 0.0f ? cell[2] < g.res[2] : cell[2] > -1);
-        }
-    }
-    if (best >= 0 && rayT < h.t && rayT >= te1 && rayT < tx1) {
-        h.t = rayT; h.u = bu; h.v = bv; h.inst = (int32_t)ii; h.tri = best;
-        return true;
-    }
-    return false;
-}
+// The traversal (TLGridHierarchyTraverser.h:45-405) is a state machine per lane, run by the
+// warp in step: a lane walks the instance grid (st 1) until a cell lists instances, the
+// boxes of all such lists are tested 32 (lane, instance) pairs at a time, a lane with a box
+// that its ray meets enters the next of them in list order (the ray in object space, the
+// object grid's DDA from the current best t, st 2), and the triangle lists of all lanes in
+// an object grid are tested together (test_lists).  Per lane the cells, instances and
+// triangles are those of the nested loops, in their order, so the hits are too; but a lane
+// deep in one object no longer holds up the lanes that are between instances (nested loops
+// per lane kept 6 of 32 lanes busy).
+//
+// What a lane needs only between objects lives in shared memory, so that the object walk
+// has the registers (33 words a lane: an odd stride, no bank conflicts).
+struct HLane {
+    float o[3], d[3], rcp[3];            // the ray
+    float tmax[3], dt[3];                // instance-grid DDA
+    int32_t left[3];
+    uint32_t stride[3], cell;
+    float t, u, v;                       // best hit so far
+    int32_t inst, tri;
+    float te, tx;                        // the entered instance: its box interval, id, grid resolution
+    int32_t ii;
+    int32_t res[3];
+};
+static_assert(sizeof(HLane) == 33 * 4, "odd word stride");
 
-// instance-grid DDA (TLGridHierarchyTraverser.h:220-405); ANY stops at the first
-// accepted hit
-template <bool ANY, bool STATS>
-__device__ void hier_trace(const HierView& H, const GridDesc& g, f3 o, f3 d, HHit& h, HCount& n) {
-    const float rcp[3] = {1.0f / d.x, 1.0f / d.y, 1.0f / d.z};
-    float t0, t1;
-    box_clip(g.bmin, g.bmax, o, rcp, &t0, &t1);
-    if (!(t1 > t0 && t1 >= 0.0f)) return;
-    f3 ep = o;
-    if (t0 >= 0.0f) {
-        const float sc = t0 + kEps;
-        ep = mk(o.x + sc * d.x, o.y + sc * d.y, o.z + sc * d.z);
-    }
-    float tmax[3];
-    int32_t cell[3];
-    bool active = true;
+#ifndef HR_HIER_REFILL
+#define HR_HIER_REFILL 12   // idle lanes that make a trace warp take new rays
+#endif
+#ifndef HR_HIER_TOP_MIN
+#define HR_HIER_TOP_MIN 6   // lanes between instances that make a warp serve them
+#endif
+#ifndef HR_HIER_CELL_STEPS
+#define HR_HIER_CELL_STEPS 3   // object cells stepped per warp step while they are empty
+#endif
+#ifndef HR_HIER_TOP_STEPS
+#define HR_HIER_TOP_STEPS 3   // instance-grid cells walked per warp step while they are empty
+#endif
+
+// DDA start of a grid walked with one-sided bounds (an entry point may lie a rounding
+// outside): t, increments, strides and steps left per axis; false when an axis is already
+// past its end.  *out: some axis is outside [0, res), so cells have to be checked.
+__device__ __forceinline__ bool onesided_start(const float* bmin, const float* cs, const float* grcp, const int32_t* res,
+                                               f3 ep, f3 o, const float* rcp, bool clamp, float* tmax, float* dt,
+                                               int32_t* left, uint32_t* stride, uint32_t* cell, bool* out) {
+    const uint32_t str[3] = {1u, (uint32_t)res[0], (uint32_t)res[0] * (uint32_t)res[1]};
+    bool ok = true;
+    *cell = 0u;
+    *out = false;
 #pragma unroll
     for (int k = 0; k < 3; ++k) {
-        const float cf = floorf((comp(ep, k) - g.bmin[k]) * g.rcp[k]);
-        const float stp = rcp[k] > 0.0f ? 1.0f : 0.0f;
-        tmax[k] = ((cf + stp) * g.cs[k] + g.bmin[k] - comp(o, k)) * rcp[k];
-        cell[k] = f2i(cf);
-        active = active && (rcp[k] > 0.0f ? cell[k] < g.res[k] : cell[k] > -1);
+        float cf = floorf((comp(ep, k) - bmin[k]) * grcp[k]);
+        const bool fwd = rcp[k] > 0.0f;
+        if (clamp) cf = fwd ? hmin((float)res[k] - 1.0f, cf) : hmax(cf, 0.0f);
+        const float stp = fwd ? 1.0f : 0.0f;
+        tmax[k] = ((cf + stp) * cs[k] + bmin[k] - comp(o, k)) * rcp[k];
+        dt[k] = cs[k] * fabsf(rcp[k]);
+        const int32_t c = f2i(cf);
+        left[k] = fwd ? (int32_t)((uint32_t)res[k] - 1u - (uint32_t)c) : c;
+        stride[k] = fwd ? str[k] : 0u - str[k];
+        *cell += (uint32_t)c * str[k];
+        ok = ok && left[k] >= 0;
+        *out = *out || left[k] >= res[k];
     }
-    const uint32_t rx = (uint32_t)g.res[0], rxy = (uint32_t)g.res[0] * (uint32_t)g.res[1];
-    while (active) {
-        if (cell[0] < g.res[0] && cell[0] > -1 && cell[1] < g.res[1] && cell[1] > -1 && cell[2] < g.res[2] &&
-            cell[2] > -1) {
-            const uint2 cr = __ldg(H.top_cells + ((uint32_t)cell[0] + (uint32_t)cell[1] * rx + (uint32_t)cell[2] * rxy));
-            if (STATS) n.top_cells++;
-            for (uint32_t it = cr.x; it < cr.y; ++it)
-                if (hier_instance<STATS>(H, __ldg(H.inst_ids + it), o, d, rcp, h, n) && ANY) return;
-        }
-        const int k = min_dim(tmax[0], tmax[1], tmax[2]);
-        float tk;
-        if (k == 0) {
-            tk = tmax[0];
-            cell[0] += rcp[0] > 0.0f ? 1 : -1;
-            tmax[0] += g.cs[0] * fabsf(rcp[0]);
-            active = h.t > tk && (rcp[0] > 0.0f ? cell[0] < g.res[0] : cell[0] > -1);
-        } else if (k == 1) {
-            tk = tmax[1];
-            cell[1] += rcp[1] > 0.0f ? 1 : -1;
-            tmax[1] += g.cs[1] * fabsf(rcp[1]);
-            active = h.t > tk && (rcp[1] > 0.0f ? cell[1] < g.res[1] : cell[1] > -1);
-        } else {
-            tk = tmax[2];
-            cell[2] += rcp[2] > 0.0f ? 1 : -1;
-            tmax[2] += g.cs[2] * fabsf(rcp[2]);
-            active = h.t > tk && (rcp[2] > 0.0f ? cell[2] < g.res[2] : cell[2] > -1);
-        }
-    }
+    return ok;
 }
 
 template <bool ANY, bool STATS>
@@ -491,42 +421,242 @@ __global__ __launch_bounds__(kTT, HR_HIER_MIN_BLOCKS) void k_hier_trace(HierView
                                                        int32_t* __restrict__ otri, float* __restrict__ ot,
                                                        float* __restrict__ ou, float* __restrict__ ov,
                                                        uint8_t* __restrict__ occ, uint32_t* __restrict__ stats,
-                                                       uint32_t* pool) {
-    const GridDesc g = *H.top;
-#if HR_HIER_WARP_POOL
-    // a warp takes 32 consecutive rays from the pool once all its lanes are done, so its
-    // lanes trace neighbouring rays together (rays listed in pixel tiles stay coherent)
-    const uint32_t lane = threadIdx.x & 31u;
+                                                       uint32_t* pool, uint32_t width) {
+    __shared__ GridDesc s_g;
+    __shared__ HLane s_lane[kTT];
+    __shared__ uint8_t s_own[kTT / 32][32];
+    for (uint32_t i = threadIdx.x; i < sizeof(GridDesc) / 4; i += kTT)
+        reinterpret_cast<uint32_t*>(&s_g)[i] = reinterpret_cast<const uint32_t*>(H.top)[i];
+    __syncthreads();
+    const GridDesc& g = s_g;
+    const uint32_t lane = threadIdx.x & 31u, lt = (1u << lane) - 1u;
+    HLane* const warp_lanes = s_lane + (threadIdx.x & ~31u);
+    HLane& L = s_lane[threadIdx.x];
+    uint8_t* const lane_of = s_own[threadIdx.x >> 5];
+    Scene s;
+    s.tris = H.tris;
+    s.prims = H.prims;
+
+    uint32_t ray = 0;
+    int st = 0;                 // 0 no ray, 1 in the instance grid, 2 in an object grid
+    bool dry = false, top_out = false, obj_out = false, fresh = false;
+    uint32_t it = 0, end = 0;   // instances of the current cell not tested yet
+    uint32_t met = 0, win = 0;  // boxes met among the 32 (or fewer) from win on, not entered yet
+    // object walk
+    f3 po = mk(0.0f, 0.0f, 0.0f), pd = mk(1.0f, 0.0f, 0.0f);
+    float otm[3] = {0.0f, 0.0f, 0.0f}, odt[3] = {0.0f, 0.0f, 0.0f};
+    int32_t oleft[3] = {0, 0, 0};
+    uint32_t ostr[3] = {0u, 0u, 0u}, ocell = 0;
+    Hit h;
+    hit_reset(h, FLT_MAX);
+    bool has = false;
+    HCount c;
     while (true) {
-        uint32_t base = 0;
-        if (lane == 0) base = atomicAdd(pool, 32u);
-        base = __shfl_sync(kFullMask, base, 0);
-        if (base >= n) break;
-        const uint32_t i = base + lane;
-        if (i >= n) continue;
-#else
-    for (uint32_t i = blockIdx.x * kTT + threadIdx.x; i < n; i += gridDim.x * kTT) {
-#endif
-        const f3 o = mk(__ldg(org + 3 * (size_t)i), __ldg(org + 3 * (size_t)i + 1), __ldg(org + 3 * (size_t)i + 2));
-        const f3 d = mk(__ldg(dir + 3 * (size_t)i), __ldg(dir + 3 * (size_t)i + 1), __ldg(dir + 3 * (size_t)i + 2));
-        HHit h;
-        h.t = ANY ? __ldg(tmax + i) : FLT_MAX;
-        h.u = 0.0f; h.v = 0.0f; h.inst = -1; h.tri = -1;
-        HCount c;
-        if (!g.error) hier_trace<ANY, STATS>(H, g, o, d, h, c);
-        if (STATS) {
-            uint32_t* st = stats + 5 * (size_t)i;
-            st[0] = c.top_cells; st[1] = c.inst_tests; st[2] = c.inst_entered; st[3] = c.obj_cells; st[4] = c.tri_tests;
+        // rays: idle lanes of the first `width` retire theirs and take the next ones together,
+        // consecutive ones, so that neighbours are traced together
+        const uint32_t need = __ballot_sync(kFullMask, st == 0 && lane < width);
+        if ((uint32_t)__popc(need) >= min(width, (uint32_t)HR_HIER_REFILL)) {
+            if (st == 0 && has) {   // results
+                if (STATS) {
+                    uint32_t* q = stats + 5 * (size_t)ray;
+                    q[0] = c.top_cells; q[1] = c.inst_tests; q[2] = c.inst_entered; q[3] = c.obj_cells; q[4] = c.tri_tests;
+                }
+                if (ANY) {
+                    occ[ray] = L.inst >= 0 ? 1 : 0;
+                } else {
+                    oinst[ray] = L.inst;
+                    otri[ray] = L.tri;
+                    ot[ray] = L.inst >= 0 ? L.t : FLT_MAX;
+                    ou[ray] = L.u;
+                    ov[ray] = L.v;
+                }
+                has = false;
+            }
+            if (!dry) {
+                uint32_t base = 0;
+                if (lane == 0) base = atomicAdd(pool, (uint32_t)__popc(need));
+                base = __shfl_sync(kFullMask, base, 0);
+                if (base >= n || n - base <= (uint32_t)__popc(need)) dry = true;
+                const uint32_t i = base + __popc(need & lt);
+                if (((need >> lane) & 1u) && base < n && i < n) {
+                    ray = i;
+                    has = true;
+                    const f3 o = mk(__ldg(org + 3 * (size_t)i), __ldg(org + 3 * (size_t)i + 1), __ldg(org + 3 * (size_t)i + 2));
+                    const f3 d = mk(__ldg(dir + 3 * (size_t)i), __ldg(dir + 3 * (size_t)i + 1), __ldg(dir + 3 * (size_t)i + 2));
+                    const float rcp[3] = {1.0f / d.x, 1.0f / d.y, 1.0f / d.z};
+                    L.o[0] = o.x; L.o[1] = o.y; L.o[2] = o.z;
+                    L.d[0] = d.x; L.d[1] = d.y; L.d[2] = d.z;
+                    L.rcp[0] = rcp[0]; L.rcp[1] = rcp[1]; L.rcp[2] = rcp[2];
+                    L.t = ANY ? __ldg(tmax + i) : FLT_MAX;
+                    L.u = 0.0f; L.v = 0.0f; L.inst = -1; L.tri = -1;
+                    c = HCount();
+                    it = end = met = 0;
+                    float t0, t1;
+                    box_clip(g.bmin, g.bmax, o, rcp, &t0, &t1);
+                    if (!g.error && t1 > t0 && t1 >= 0.0f) {
+                        f3 ep = o;
+                        if (t0 >= 0.0f) {
+                            const float sc = t0 + kEps;
+                            ep = mk(o.x + sc * d.x, o.y + sc * d.y, o.z + sc * d.z);
+                        }
+                        if (onesided_start(g.bmin, g.cs, g.rcp, g.res, ep, o, rcp, false, L.tmax, L.dt, L.left, L.stride,
+                                           &L.cell, &top_out))
+                            st = 1;
+                        fresh = true;
+                    }
+                }
+            }
+            if (!__any_sync(kFullMask, has)) break;
         }
-        if (ANY) {
-            occ[i] = h.inst >= 0 ? 1 : 0;
-        } else {
-            oinst[i] = h.inst;
-            otri[i] = h.tri;
-            ot[i] = h.inst >= 0 ? h.t : FLT_MAX;
-            ou[i] = h.u;
-            ov[i] = h.v;
+
+        // lanes between instances wait until HR_HIER_TOP_MIN of them do, or none is in an object
+        const uint32_t tops = __ballot_sync(kFullMask, st == 1);
+        if (tops && ((uint32_t)__popc(tops) >= HR_HIER_TOP_MIN || !__any_sync(kFullMask, st == 2))) {
+            // instance grid: lanes that are through with their cell's list walk on to the next
+            // cell with one (fresh: the cell they stand in has not been looked at)
+            if (st == 1 && met == 0u && it >= end) {
+                for (int k = 0; k < HR_HIER_TOP_STEPS; ++k) {
+                    if (!fresh) {
+                        float tk;
+                        uint32_t cell = L.cell;
+                        const bool inside = dda_step(L.tmax, L.dt, cell, L.stride, L.left, &tk);
+                        L.cell = cell;
+                        if (!(L.t > tk && inside)) {
+                            st = 0;
+                            break;
+                        }
+                    }
+                    fresh = false;
+                    if (top_out) {
+                        if (L.left[0] >= g.res[0] || L.left[1] >= g.res[1] || L.left[2] >= g.res[2]) continue;
+                        top_out = false;
+                    }
+                    if (STATS) c.top_cells++;
+                    const uint2 cr = __ldg(H.top_cells + L.cell);
+                    it = cr.x;
+                    end = cr.y;
+                    if (cr.y > cr.x) break;
+                }
+            }
+            __syncwarp();
+
+            // the boxes of the lists, 32 (lane, instance) pairs per round; a lane's window is at
+            // most 32 instances
+            const uint32_t nw = st == 1 && met == 0u ? min(end - it, 32u) : 0u;
+            const uint32_t ne = __ballot_sync(kFullMask, nw != 0u);
+            if (ne) {
+                uint32_t incl = nw;
+    #pragma unroll
+                for (int off = 1; off < 32; off <<= 1) {
+                    const uint32_t x = __shfl_up_sync(kFullMask, incl, off);
+                    if (lane >= (uint32_t)off) incl += x;
+                }
+                const uint32_t total = __shfl_sync(kFullMask, incl, 31), excl = incl - nw;
+                if (nw != 0u) lane_of[__popc(ne & lt)] = (uint8_t)lane;
+                __syncwarp();
+                if (nw != 0u) win = it;
+                it += nw;
+                if (STATS) c.inst_tests += nw;
+                const uint32_t rel = win - excl;
+                uint32_t started = 0xffffffffu;
+                for (uint32_t base = 0; base < total; base += 32u) {
+                    const uint32_t j = base + lane, rs = excl - base;
+                    const uint32_t heads = __reduce_or_sync(kFullMask, (nw != 0u && rs < 32u) ? 1u << rs : 0u);
+                    const int own = lane_of[started + __popc(heads & (0xffffffffu >> (31u - lane)))];
+                    started += __popc(heads);
+                    const uint32_t at = shfl(rel, own) + j;
+                    bool in = false;
+                    if (j < total) {
+                        const HLane& Q = warp_lanes[own];
+                        const HierInst* I = H.inst + __ldg(H.inst_ids + at);
+                        const float4 lo = __ldg(&I->lo), hi = __ldg(&I->hi);
+                        const float blo[3] = {lo.x, lo.y, lo.z}, bhi[3] = {hi.x, hi.y, hi.z};
+                        float te, tx;
+                        box_clip(blo, bhi, mk(Q.o[0], Q.o[1], Q.o[2]), Q.rcp, &te, &tx);
+                        in = tx > te && tx >= 0.0f && te < Q.t;
+                    }
+                    const uint32_t hm = __ballot_sync(kFullMask, in);
+                    const uint32_t lo = excl > base ? min(rs, 32u) : 0u, hi = incl > base ? min(incl - base, 32u) : 0u;
+                    if (lo < hi) met |= ((hm >> lo) & (0xffffffffu >> (32u - (hi - lo)))) << (base + lo - excl);
+                }
+                __syncwarp();
+            }
+
+            // enter the next instance met (its box interval is checked again: the best t may
+            // have come closer since the boxes were tested)
+            if (st == 1 && met != 0u) {
+                const uint32_t ii = __ldg(H.inst_ids + win + (uint32_t)(__ffs(met) - 1));
+                met &= met - 1u;
+                const HierInst* I = H.inst + ii;
+                const float4 lo = __ldg(&I->lo), hi = __ldg(&I->hi);
+                const float blo[3] = {lo.x, lo.y, lo.z}, bhi[3] = {hi.x, hi.y, hi.z};
+                const f3 o = mk(L.o[0], L.o[1], L.o[2]), d = mk(L.d[0], L.d[1], L.d[2]);
+                float te, tx;
+                box_clip(blo, bhi, o, L.rcp, &te, &tx);
+                const float best = L.t;
+                if (te < best) {
+                    if (STATS) c.inst_entered++;
+                    L.te = te; L.tx = tx; L.ii = (int32_t)ii;
+                    const float4 r0 = __ldg(&I->r0), r1 = __ldg(&I->r1), r2 = __ldg(&I->r2);
+                    po = mk(r0.x * o.x + r0.y * o.y + r0.z * o.z + r0.w, r1.x * o.x + r1.y * o.y + r1.z * o.z + r1.w,
+                            r2.x * o.x + r2.y * o.y + r2.z * o.z + r2.w);
+                    pd = mk(r0.x * d.x + r0.y * d.y + r0.z * d.z, r1.x * d.x + r1.y * d.y + r1.z * d.z,
+                            r2.x * d.x + r2.y * d.y + r2.z * d.z);
+                    const float rt[3] = {1.0f / pd.x, 1.0f / pd.y, 1.0f / pd.z};
+                    const HierObj& O = H.objs[__float_as_uint(lo.w)];
+                    float oe, ox;
+                    box_clip(O.bmin, O.bmax, po, rt, &oe, &ox);
+                    f3 ep = po;
+                    if (oe >= 0.0f) {
+                        const float sc = oe + kEps;
+                        ep = mk(po.x + sc * pd.x, po.y + sc * pd.y, po.z + sc * pd.z);
+                    }
+                    if (onesided_start(O.bmin, O.cs, O.rcp, O.res, ep, po, rt, true, otm, odt, oleft, ostr, &ocell, &obj_out) &&
+                        ox > oe && ox >= 0.0f && oe < best) {
+                        ocell += O.cell_off;
+                        L.res[0] = O.res[0]; L.res[1] = O.res[1]; L.res[2] = O.res[2];
+                        hit_reset(h, best);
+                        st = 2;
+                    }
+                }
+            }
+
         }
+
+        // object grids: the current cells' lists, then on to the next cell with one
+        uint2 cr = make_uint2(0u, 0u);
+        if (st == 2) {
+            if (obj_out) obj_out = oleft[0] >= L.res[0] || oleft[1] >= L.res[1] || oleft[2] >= L.res[2];
+            if (!obj_out) {
+                cr = __ldg(H.obj_cells + ocell);
+                if (STATS) c.obj_cells++;
+            }
+        }
+        test_lists<kHitClosest, STATS>(s, po, pd, cr.x, cr.y, false, h);
+        if (st == 2) {
+            bool done = false;
+            for (int k = 1;; ++k) {
+                float tk;
+                const bool inside = dda_step(otm, odt, ocell, ostr, oleft, &tk);
+                if (!(inside && h.t > tk)) {
+                    done = true;
+                    break;
+                }
+                if (k >= HR_HIER_CELL_STEPS || obj_out) break;
+                const uint2 nx = __ldg(H.obj_cells + ocell);
+                if (nx.y > nx.x) break;
+                if (STATS) c.obj_cells++;
+            }
+            if (done) {
+                st = 1;
+                if (STATS) c.tri_tests += h.tests;
+                if (h.hit && h.t < L.t && h.t >= L.te && h.t < L.tx) {
+                    L.t = h.t; L.u = h.u; L.v = h.v; L.inst = L.ii; L.tri = (int32_t)h.tri;
+                    if (ANY) st = 0;
+                }
+            }
+        }
+        __syncwarp();
     }
 }
 
@@ -568,20 +698,16 @@ int grid_of(const hr_ctx* c, uint64_t n, int bt) {
     return (int)std::max<uint64_t>(1, std::min(b, cap));
 }
 
-// blocks of the trace launch: resident blocks on every SM with the warp ray pool,
-// enough blocks for one ray per thread otherwise
-template <bool ANY, bool STATS>
-int hier_grid(hr_ctx* c, uint32_t n) {
-    const int want = grid_of(c, n, kTT);
-    if (!HR_HIER_WARP_POOL) return want;
-    int nb = 0;
-    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, k_hier_trace<ANY, STATS>, kTT, 0) != cudaSuccess || nb < 1) {
-        cudaGetLastError();
-        nb = 1;
-    }
-    return std::max(1, std::min(want, nb * c->num_sms));
+// Blocks of the trace launch, all resident at once (the launch bounds allow
+// HR_HIER_MIN_BLOCKS per SM), and the rays a warp holds at a time: 32, or a smaller power of
+// two (at least 8) while n rays do not fill the warps (320 x 160 rays 0.176 -> 0.123 ms).
+int hier_grid(const hr_ctx* c, uint32_t n, uint32_t* width) {
+    const uint64_t blocks = (uint64_t)HR_HIER_MIN_BLOCKS * c->num_sms, wpb = kTT / 32;
+    *width = 32u;
+    while (*width > 8u && n < blocks * wpb * *width) *width /= 2u;
+    const uint64_t want = ((uint64_t)n + *width * wpb - 1) / (*width * wpb);
+    return (int)std::max<uint64_t>(1, std::min(want, blocks));
 }
-
 
 // level two: object grids
 int build_objects(hr_hier* h) {
@@ -666,7 +792,7 @@ int build_instances(hr_hier* h) {
         (rc = ensure(c, B.scan_partials, sizeof(uint32_t) * (scan_partials_words(std::max(h->ninst, h->nobj)) + 2))))
         return rc;
     c->launches += 2;
-    k_hier_top_setup<<<1, kBT, 0, s>>>(h->inst.as<HierInst>(), h->ninst, h->top_density, td);
+    k_hier_top_setup<<<1, kTopThreads, 0, s>>>(h->inst.as<HierInst>(), h->ninst, h->top_density, td);
     k_hier_inst_count<<<grid_of(c, h->ninst, 256), 256, 0, s>>>(h->inst.as<HierInst>(), h->ninst, td,
                                                                 h->icnt.as<uint32_t>());
     if ((rc = exclusive_scan_u32(c, h->icnt.as<uint32_t>(), words + 5, h->ninst, words + 2,
@@ -913,11 +1039,13 @@ hr_status hr_hier_trace_rays_device(hr_hier* h, const float* org, const float* d
     DeviceGuard dg(c->device);
     c->launches += 1;
     uint32_t* pool = h->words.as<uint32_t>() + 7;
+    uint32_t width;
+    const int nb = hier_grid(c, n, &width);
     if (cudaMemsetAsync(pool, 0, 4, c->stream) != cudaSuccess)
         return (hr_status)cuda_check(c, cudaGetLastError(), "hier ray pool");
-    k_hier_trace<false, false><<<hier_grid<false, false>(c, n), kTT, 0, c->stream>>>(view(h), org, dir, nullptr, n,
+    k_hier_trace<false, false><<<nb, kTT, 0, c->stream>>>(view(h), org, dir, nullptr, n,
                                                                                     inst_id, tri_id, t, u, v, nullptr,
-                                                                                    nullptr, pool);
+                                                                                    nullptr, pool, width);
     return (hr_status)cuda_check(c, cudaGetLastError(), "hier trace launch");
 }
 
@@ -930,11 +1058,13 @@ hr_status hr_hier_trace_stats_device(hr_hier* h, const float* org, const float* 
     DeviceGuard dg(c->device);
     c->launches += 1;
     uint32_t* pool = h->words.as<uint32_t>() + 7;
+    uint32_t width;
+    const int nb = hier_grid(c, n, &width);
     if (cudaMemsetAsync(pool, 0, 4, c->stream) != cudaSuccess)
         return (hr_status)cuda_check(c, cudaGetLastError(), "hier ray pool");
-    k_hier_trace<false, true><<<hier_grid<false, true>(c, n), kTT, 0, c->stream>>>(view(h), org, dir, nullptr, n,
+    k_hier_trace<false, true><<<nb, kTT, 0, c->stream>>>(view(h), org, dir, nullptr, n,
                                                                                   inst_id, tri_id, t, u, v, nullptr,
-                                                                                  stats, pool);
+                                                                                  stats, pool, width);
     return (hr_status)cuda_check(c, cudaGetLastError(), "hier trace launch");
 }
 
@@ -987,9 +1117,11 @@ hr_status hr_hier_occluded(hr_hier* h, const float* org, const float* dir, const
         return (hr_status)rc;
     c->launches += 1;
     uint32_t* pool = h->words.as<uint32_t>() + 7;
+    uint32_t width;
+    const int nb = hier_grid(c, n, &width);
     if ((rc = cuda_check(c, cudaMemsetAsync(pool, 0, 4, s), "hier ray pool"))) return (hr_status)rc;
-    k_hier_trace<true, false><<<hier_grid<true, false>(c, n), kTT, 0, s>>>(view(h), dorg, ddir, dtm, n, nullptr, nullptr,
-                                                                          nullptr, nullptr, nullptr, docc, nullptr, pool);
+    k_hier_trace<true, false><<<nb, kTT, 0, s>>>(view(h), dorg, ddir, dtm, n, nullptr, nullptr,
+                                                                          nullptr, nullptr, nullptr, docc, nullptr, pool, width);
     if ((rc = cuda_check(c, cudaGetLastError(), "hier occluded launch")) ||
         (rc = cuda_check(c, cudaMemcpyAsync(occluded, docc, n, cudaMemcpyDeviceToHost, s), "occluded")))
         return (hr_status)rc;
