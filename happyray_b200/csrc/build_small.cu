@@ -20,7 +20,7 @@
 //      once, so this is the order the stable sort of the triangle-ordered pairs gives)
 // Phases 5-7 replace the radix sort and the range pass when no cell holds more than
 // kCountListMax triangles; otherwise (decided alike in every block from the phase-4
-// maxima) the launch runs the pipeline's stable LSD radix passes (sort.cu) and cell ranges.
+// maxima) the launch runs stable LSD radix passes (radix_tile.cuh) and cell ranges.
 // Each phase computes what the pipeline computes, so the grid is bit-identical to it.
 // Values written by one phase and read by another are read with L2-coherent loads (the
 // read-only path may hold stale lines within a launch); block b keeps its triangles
@@ -503,13 +503,13 @@ __global__ __launch_bounds__(kBT, 3) void k_build_ug_small(SmallUG P) {
         uint32_t* dv = last ? P.prims : (pp % 2 == 0 ? P.vals_b : P.vals_a);
         const int shift = pp * P.db;
         for (uint32_t tile = b; tile < ntiles; tile += G)
-            radix_upsweep_tile<true>(src_k, npairs, shift, mask, P.tile_hist, ntiles, tile);
+            radix_upsweep_tile(src_k, npairs, shift, mask, P.tile_hist, ntiles, tile);
         if (!grid_barrier(P.bar, P.d)) return;
         for (uint32_t dg = b; dg <= mask; dg += G)
-            radix_scan_row<kBT, true>(P.tile_hist + (size_t)dg * ntiles, ntiles, P.row_total + dg);
+            radix_scan_row<kBT>(P.tile_hist + (size_t)dg * ntiles, ntiles, P.row_total + dg);
         if (!grid_barrier(P.bar, P.d)) return;
         for (uint32_t tile = b; tile < ntiles; tile += G)
-            radix_downsweep_tile<true>(src_k, src_v, dk, dv, npairs, shift, mask, P.tile_hist, ntiles, P.row_total,
+            radix_downsweep_tile(src_k, src_v, dk, dv, npairs, shift, mask, P.tile_hist, ntiles, P.row_total,
                                        tile);
         if (!grid_barrier(P.bar, P.d)) return;
         src_k = dk;

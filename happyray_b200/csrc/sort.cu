@@ -4,9 +4,8 @@
 // Replaces the reference's CUB wrappers: ExclusiveScan (Scan.cu:39-58) and RadixSort
 // (Sort.cu:31-53, cub::DeviceRadixSort::SortPairs over uint32 keys/values).
 //
-// Design: reduce-then-scan in every pass (upsweep tile histograms, one CTA per digit
-// scans its row of tile counts, downsweep ranks and scatters), so no kernel waits on
-// another CTA and nothing spins.  All element counts are read from device memory, so
+// Design: reduce-then-scan in every pass (tile digit counts, their scan over the tiles,
+// rank and scatter), so no kernel waits on another CTA and nothing spins.  All element counts are read from device memory, so
 // the whole pipeline is enqueued without a host round trip; grids are sized from the
 // host-side capacity and surplus CTAs exit at once.
 #include "hr_internal.h"
@@ -112,25 +111,213 @@ __global__ __launch_bounds__(kThreads) void k_scan_apply(T* data, const uint32_t
 }
 
 // ----------------------------------------------------------------------------------
-// radix sort kernels
+// radix sort kernels: tiles of 256 x ITEMS keys, digits of up to BITS bits.  Tile counts are
+// stored tile by tile (nd = 2^digit bits words each), so that a tile writes and reads its
+// counts in one run.  (The single-launch build keeps the steps of radix_tile.cuh, whose
+// tiles of 2048 keys suit its few pairs.)
 
-__global__ __launch_bounds__(kThreads) void k_radix_upsweep(const uint32_t* __restrict__ keys, const uint32_t* d_count,
-                                                            int shift, uint32_t mask, uint32_t* tile_hist,
-                                                            uint32_t ntiles_cap) {
-    radix_upsweep_tile<false>(keys, *d_count, shift, mask, tile_hist, ntiles_cap, blockIdx.x);
+// The run of equal digits among neighbouring lanes that this lane begins, as a lane mask; 0
+// when the lane before it holds the same digit.  A mesh's pairs come with many equal
+// digits side by side, and a run then costs one shared-memory atomic.
+__device__ __forceinline__ uint32_t digit_run(uint32_t dig) {
+    const uint32_t lane = threadIdx.x & 31u;
+    const uint32_t prev = __shfl_up_sync(kFullMask, dig, 1);
+    const bool head = lane == 0u || prev != dig;
+    const uint32_t after = __ballot_sync(kFullMask, head) & (0xfffffffeu << lane);
+    return head ? ((after & (0u - after)) - 1u) & (0xffffffffu << lane) : 0u;
 }
 
-// one CTA per digit: exclusive scan of its row of tile counts, row total out
-__global__ __launch_bounds__(1024) void k_radix_scan(uint32_t* tile_hist, uint32_t ntiles_cap, uint32_t* row_total) {
-    radix_scan_row<1024>(tile_hist + (size_t)blockIdx.x * ntiles_cap, ntiles_cap, row_total + blockIdx.x);
+// tile digit counts, an add per run of equal digits
+template <int BITS, int ITEMS>
+__global__ __launch_bounds__(kThreads) void k_radix_count(const uint32_t* __restrict__ keys, const uint32_t* d_count,
+                                                          int shift, uint32_t mask, uint32_t* __restrict__ tile_hist) {
+    __shared__ uint32_t h[1 << BITS];
+    const uint32_t n = *d_count;
+    const size_t base = (size_t)blockIdx.x * (kThreads * ITEMS);
+    if (base >= n) return;
+    for (uint32_t d = threadIdx.x; d <= mask; d += kThreads) h[d] = 0u;
+    uint32_t key[ITEMS];
+#pragma unroll
+    for (int k = 0; k < ITEMS; ++k) {
+        const size_t i = base + threadIdx.x + (size_t)k * kThreads;
+        key[k] = i < n ? __ldg(keys + i) : 0u;
+    }
+    __syncthreads();
+#pragma unroll
+    for (int k = 0; k < ITEMS; ++k) {
+        const bool valid = base + threadIdx.x + (size_t)k * kThreads < n;
+        const uint32_t dig = valid ? (key[k] >> shift) & mask : 0xffffffffu, run = digit_run(dig);
+        if (valid && run) atomicAdd(&h[dig], (uint32_t)__popc(run));
+    }
+    __syncthreads();
+    uint32_t* out = tile_hist + (size_t)blockIdx.x * (mask + 1u);
+    for (uint32_t d = threadIdx.x; d <= mask; d += kThreads) out[d] = h[d];
 }
 
-__global__ __launch_bounds__(kThreads) void k_radix_downsweep(
+// exclusive scan of the tile counts of each digit over the tiles, in place, and the digit
+// totals: a block takes 32 digits (a lane each), its warps consecutive runs of tiles
+template <int ITEMS>
+__global__ __launch_bounds__(1024) void k_radix_scan(uint32_t* __restrict__ tile_hist, const uint32_t* d_count, uint32_t nd,
+                                                     uint32_t* __restrict__ row_total) {
+    __shared__ uint32_t s[32][33];
+    const uint32_t ntiles = (uint32_t)(((size_t)*d_count + kThreads * ITEMS - 1) / (kThreads * ITEMS));
+    const uint32_t lane = threadIdx.x & 31u, w = threadIdx.x >> 5, d = blockIdx.x * 32u + lane;
+    const uint32_t chunk = (ntiles + 31u) / 32u, t0 = min(w * chunk, ntiles), t1 = min(t0 + chunk, ntiles);
+    uint32_t* col = tile_hist + d;
+    constexpr uint32_t kRows = 16;   // loads in flight per thread
+    uint32_t sum = 0;
+    if (d < nd)
+        for (uint32_t t = t0; t < t1; t += kRows) {
+            uint32_t x[kRows];
+#pragma unroll
+            for (uint32_t k = 0; k < kRows; ++k) x[k] = t + k < t1 ? __ldcg(col + (size_t)(t + k) * nd) : 0u;
+#pragma unroll
+            for (uint32_t k = 0; k < kRows; ++k) sum += x[k];
+        }
+    s[w][lane] = sum;
+    __syncthreads();
+    uint32_t run = 0;
+    for (uint32_t k = 0; k < w; ++k) run += s[k][lane];
+    if (d < nd) {
+        if (w == 31u) row_total[d] = run + sum;
+        for (uint32_t t = t0; t < t1; t += kRows) {
+            uint32_t x[kRows];
+#pragma unroll
+            for (uint32_t k = 0; k < kRows; ++k) x[k] = t + k < t1 ? __ldcg(col + (size_t)(t + k) * nd) : 0u;
+#pragma unroll
+            for (uint32_t k = 0; k < kRows; ++k) {
+                if (t + k < t1) col[(size_t)(t + k) * nd] = run;
+                run += x[k];
+            }
+        }
+    }
+}
+
+// stable rank and scatter of a tile: a key goes to its digit's start (the totals scanned
+// here) plus the tile's scanned count plus its rank among the tile's keys of the digit.
+//
+// Ranks within a warp's row of 32 keys come alternately from two pipes, because each alone
+// bounds the kernel: a match of the digits holds its pipe for 32 cycles a warp, and the
+// other way, each run of equal digits oring its lanes into the digit's word (whose set bits
+// below a lane are its rank), costs about 15 shared-memory cycles.  All three passes over
+// 4.87M leaf pairs of a 2M-triangle mesh / 4.8M random keys of 23 bits: every row by match
+// 203 / 258 us, by oring 219 / 218, in turn 205 / 222 (tiles of 2048 keys 209 / 239; the kernel
+// before, by match over 512 counters, 209 / 337).  511k pairs: tiles of 2048 keys 92 us, 4096
+// 103; 158k 52 and 62; 2.1M 134 and 130, so the line lies where both sizes fill the GPU.
+template <int BITS, int ITEMS>
+__global__ __launch_bounds__(kThreads, 4) void k_radix_scatter(
     const uint32_t* __restrict__ keys_in, const uint32_t* __restrict__ vals_in, uint32_t* __restrict__ keys_out,
     uint32_t* __restrict__ vals_out, const uint32_t* d_count, int shift, uint32_t mask,
-    const uint32_t* __restrict__ tile_hist, uint32_t ntiles_cap, const uint32_t* __restrict__ row_total) {
-    radix_downsweep_tile<false>(keys_in, vals_in, keys_out, vals_out, *d_count, shift, mask, tile_hist, ntiles_cap,
-                                row_total, blockIdx.x);
+    const uint32_t* __restrict__ tile_hist, const uint32_t* __restrict__ row_total) {
+    constexpr int ND = 1 << BITS, TILE = kThreads * ITEMS, DPT = ND / kThreads > 0 ? ND / kThreads : 1;
+    extern __shared__ __align__(16) unsigned char s_raw[];   // ranks, then the sorted tile
+    uint2(*s_rank)[ND] = reinterpret_cast<uint2(*)[ND]>(s_raw);
+    uint2* s_kv = reinterpret_cast<uint2*>(s_raw);
+    __shared__ uint32_t s_goff[ND];   // digit's place in the output, minus its place in the tile
+
+    const uint32_t n = *d_count;
+    const size_t base = (size_t)blockIdx.x * TILE;
+    if (base >= n) return;
+    const uint32_t nvalid = (uint32_t)min((size_t)TILE, n - base);
+    const uint32_t lane = threadIdx.x & 31u, w = threadIdx.x >> 5, lt = (1u << lane) - 1u;
+    uint32_t key[ITEMS];
+    const uint32_t li0 = w * 32u * ITEMS + lane;
+#pragma unroll
+    for (int r = 0; r < ITEMS; ++r) {
+        const uint32_t li = li0 + (uint32_t)r * 32u;
+        key[r] = li < nvalid ? __ldg(keys_in + base + li) : 0u;
+    }
+    for (uint32_t i = threadIdx.x; i < (uint32_t)(kWarps * ND); i += kThreads) (&s_rank[0][0])[i] = make_uint2(0u, 0u);
+    // digit starts: exclusive scan of the totals (DPT consecutive digits per thread)
+    {
+        uint32_t t[DPT], sum = 0, all;
+#pragma unroll
+        for (int j = 0; j < DPT; ++j) {
+            const uint32_t d = threadIdx.x * DPT + j;
+            t[j] = d <= mask ? __ldg(row_total + d) : 0u;
+            sum += t[j];
+        }
+        uint32_t ex = block_excl_scan<uint32_t, kThreads>(sum, &all);
+        const uint32_t* col = tile_hist + (size_t)blockIdx.x * (mask + 1u);
+#pragma unroll
+        for (int j = 0; j < DPT; ++j) {
+            const uint32_t d = threadIdx.x * DPT + j;
+            if (d <= mask) s_goff[d] = ex + __ldg(col + d);
+            ex += t[j];
+        }
+    }
+    __syncthreads();
+    uint32_t rank[ITEMS];
+    uint2* const mine = s_rank[w];
+#pragma unroll
+    for (int r = 0; r < ITEMS; ++r) {
+        const bool valid = li0 + (uint32_t)r * 32u < nvalid;
+        const uint32_t dig = (key[r] >> shift) & mask;
+        if (r & 1) {
+            const uint32_t run = digit_run(valid ? dig : 0xffffffffu);
+            if (valid && run) atomicOr(&mine[dig].x, run);
+            __syncwarp();
+            uint2 q = make_uint2(0u, 0u);
+            if (valid) q = mine[dig];
+            rank[r] = q.y + __popc(q.x & lt);
+            __syncwarp();
+            if (valid && (q.x & lt) == 0u) mine[dig] = make_uint2(0u, q.y + __popc(q.x));   // the digit's first lane
+            __syncwarp();
+        } else {
+            const uint32_t peers = __match_any_sync(kFullMask, valid ? dig : 0xffffffffu);
+            uint32_t b = 0;
+            if (valid) b = mine[dig].y;
+            rank[r] = b + __popc(peers & lt);
+            __syncwarp();
+            if (valid && (peers & lt) == 0u) mine[dig].y = b + __popc(peers);
+            __syncwarp();
+        }
+    }
+    __syncthreads();
+    // per digit: the tile-local start plus the prefix over the warps, where its keys rank
+    // from; and what leads from there to its place in the output
+    {
+        uint32_t c[DPT][kWarps], sum = 0, all;
+#pragma unroll
+        for (int j = 0; j < DPT; ++j) {
+            const uint32_t d = threadIdx.x * DPT + j;
+#pragma unroll
+            for (int ww = 0; ww < kWarps; ++ww) {
+                c[j][ww] = d <= mask ? s_rank[ww][d].y : 0u;
+                sum += c[j][ww];
+            }
+        }
+        uint32_t ex = block_excl_scan<uint32_t, kThreads>(sum, &all);
+#pragma unroll
+        for (int j = 0; j < DPT; ++j) {
+            const uint32_t d = threadIdx.x * DPT + j;
+            if (d <= mask) {
+                s_goff[d] -= ex;
+#pragma unroll
+                for (int ww = 0; ww < kWarps; ++ww) {
+                    s_rank[ww][d].y = ex;
+                    ex += c[j][ww];
+                }
+            }
+        }
+    }
+    __syncthreads();
+#pragma unroll
+    for (int r = 0; r < ITEMS; ++r)
+        if (li0 + (uint32_t)r * 32u < nvalid) rank[r] += mine[(key[r] >> shift) & mask].y;
+    __syncthreads();   // the ranks are read: the buffer takes the sorted tile
+#pragma unroll
+    for (int r = 0; r < ITEMS; ++r)
+        if (li0 + (uint32_t)r * 32u < nvalid)
+            s_kv[rank[r]] = make_uint2(key[r], __ldg(vals_in + base + li0 + (uint32_t)r * 32u));
+    __syncthreads();
+#pragma unroll 4
+    for (uint32_t j = threadIdx.x; j < nvalid; j += kThreads) {
+        const uint2 q = s_kv[j];
+        const uint32_t at = s_goff[(q.x >> shift) & mask] + j;
+        keys_out[at] = q.x;
+        vals_out[at] = q.y;
+    }
 }
 
 }  // namespace
@@ -214,6 +401,7 @@ static void radix_plan(int key_bits, int max_db, int* passes, int* db) {
     *db = (key_bits + *passes - 1) / *passes;
 }
 
+constexpr size_t kWideTileKeys = 148 * 4 * 2048;   // from this many keys on, tiles of 4096 keys
 constexpr int kMaxDigitBits = 9;   // context sorts; the allocation-free sort keeps 8 (its static scratch)
 
 int radix_sort_passes(int key_bits) {
@@ -222,12 +410,56 @@ int radix_sort_passes(int key_bits) {
     return passes;
 }
 
+// keys per thread of a sort over up to cap_count keys: tiles of 4096 keys halve the counts
+// and the per-tile work, but need more keys to fill the GPU (see k_radix_scatter)
+static int radix_items(size_t cap_count) { return cap_count >= kWideTileKeys ? 16 : 8; }
+
 size_t radix_tile_hist_words(size_t cap_count, int key_bits) {
     int passes, db;
     radix_plan(key_bits, kMaxDigitBits, &passes, &db);
-    size_t ntiles = (cap_count + kTile - 1) / kTile;
+    size_t ntiles = (cap_count + kTile - 1) / kTile;   // the smaller tiles
     if (ntiles == 0) ntiles = 1;
     return ntiles * ((size_t)1 << db);
+}
+
+// one pass: counts, scan, scatter
+template <int BITS, int ITEMS>
+static cudaError_t radix_pass(const uint32_t* sk, const uint32_t* sv, uint32_t* dk, uint32_t* dv, const uint32_t* d_count,
+                              size_t cap_count, int shift, uint32_t mask, uint32_t* tile_hist, uint32_t* row_total,
+                              cudaStream_t s) {
+    constexpr size_t rank = sizeof(uint2) * kWarps * (1 << BITS), sort = sizeof(uint32_t) * 2 * kThreads * ITEMS;
+    constexpr size_t smem = rank > sort ? rank : sort;
+    const uint32_t ntiles = (uint32_t)((cap_count + kThreads * ITEMS - 1) / (kThreads * ITEMS));
+    k_radix_count<BITS, ITEMS><<<ntiles, kThreads, 0, s>>>(sk, d_count, shift, mask, tile_hist);
+    k_radix_scan<ITEMS><<<(mask + 32u) / 32u, 1024, 0, s>>>(tile_hist, d_count, mask + 1u, row_total);
+    k_radix_scatter<BITS, ITEMS><<<ntiles, kThreads, smem, s>>>(sk, sv, dk, dv, d_count, shift, mask, tile_hist, row_total);
+    return cudaGetLastError();
+}
+
+// all passes of a plan with digits of at most max_db bits
+static cudaError_t radix_passes(const uint32_t* keys_in, const uint32_t* vals_in, uint32_t* keys_tmp, uint32_t* vals_tmp,
+                                uint32_t* keys_out, uint32_t* vals_out, const uint32_t* d_count, size_t cap_count,
+                                int key_bits, int max_db, uint32_t* tile_hist, uint32_t* row_total, cudaStream_t s,
+                                uint64_t* launches) {
+    int passes, db;
+    radix_plan(key_bits, max_db, &passes, &db);
+    const uint32_t mask = (1u << db) - 1u;
+    if (cap_count == 0) return cudaSuccess;
+    const uint32_t* sk = keys_in;
+    const uint32_t* sv = vals_in;
+    for (int p = 0; p < passes; ++p) {
+        const bool last = p == passes - 1;
+        uint32_t* dk = last ? keys_out : ((p % 2 == 0) ? keys_tmp : const_cast<uint32_t*>(keys_in));
+        uint32_t* dv = last ? vals_out : ((p % 2 == 0) ? vals_tmp : const_cast<uint32_t*>(vals_in));
+        auto pass = db <= 8 ? (radix_items(cap_count) == 16 ? radix_pass<8, 16> : radix_pass<8, 8>)
+                            : (radix_items(cap_count) == 16 ? radix_pass<9, 16> : radix_pass<9, 8>);
+        const cudaError_t e = pass(sk, sv, dk, dv, d_count, cap_count, p * db, mask, tile_hist, row_total, s);
+        if (e != cudaSuccess) return e;
+        if (launches) *launches += 3;
+        sk = dk;
+        sv = dv;
+    }
+    return cudaSuccess;
 }
 
 int radix_sort_pairs(hr_ctx* c, const uint32_t* keys_in, const uint32_t* vals_in,
@@ -238,27 +470,8 @@ int radix_sort_pairs(hr_ctx* c, const uint32_t* keys_in, const uint32_t* vals_in
     if (radix_tile_hist_words(cap_count, key_bits) * sizeof(uint32_t) > tile_hist_bytes)
         return set_error(c, 4, "radix sort: histogram of %zu bytes is too small for %zu keys of %d bits",
                          tile_hist_bytes, cap_count, key_bits);
-    int passes, db;
-    radix_plan(key_bits, kMaxDigitBits, &passes, &db);
-    const uint32_t mask = (1u << db) - 1u;
-    const uint32_t ntiles = (uint32_t)((cap_count + kTile - 1) / kTile);
-    if (ntiles == 0) return 0;
-    const uint32_t* src_k = keys_in;
-    const uint32_t* src_v = vals_in;
-    for (int p = 0; p < passes; ++p) {
-        const bool last = p == passes - 1;
-        uint32_t* dk = last ? keys_out : ((p % 2 == 0) ? keys_tmp : const_cast<uint32_t*>(keys_in));
-        uint32_t* dv = last ? vals_out : ((p % 2 == 0) ? vals_tmp : const_cast<uint32_t*>(vals_in));
-        const int shift = p * db;
-        c->launches += 3;
-        k_radix_upsweep<<<ntiles, kThreads, 0, s>>>(src_k, d_count, shift, mask, tile_hist, ntiles);
-        k_radix_scan<<<mask + 1, 1024, 0, s>>>(tile_hist, ntiles, row_total);
-        k_radix_downsweep<<<ntiles, kThreads, 0, s>>>(src_k, src_v, dk, dv, d_count, shift, mask, tile_hist,
-                                                      ntiles, row_total);
-        src_k = dk;
-        src_v = dv;
-    }
-    return cuda_check(c, cudaGetLastError(), "radix_sort_pairs");
+    return cuda_check(c, radix_passes(keys_in, vals_in, keys_tmp, vals_tmp, keys_out, vals_out, d_count, cap_count, key_bits,
+                                      kMaxDigitBits, tile_hist, row_total, s, &c->launches), "radix_sort_pairs");
 }
 
 // Same pass sequence as radix_sort_pairs, without a context (no status text, no launch
@@ -267,26 +480,8 @@ cudaError_t radix_sort_pairs_raw(const uint32_t* keys_in, const uint32_t* vals_i
                                  uint32_t* vals_tmp, uint32_t* keys_out, uint32_t* vals_out,
                                  const uint32_t* d_count, size_t cap_count, int key_bits, uint32_t* tile_hist,
                                  uint32_t* row_total, cudaStream_t s) {
-    int passes, db;
-    radix_plan(key_bits, 8, &passes, &db);
-    const uint32_t mask = (1u << db) - 1u;
-    const uint32_t ntiles = (uint32_t)((cap_count + kTile - 1) / kTile);
-    if (ntiles == 0) return cudaSuccess;
-    const uint32_t* src_k = keys_in;
-    const uint32_t* src_v = vals_in;
-    for (int p = 0; p < passes; ++p) {
-        const bool last = p == passes - 1;
-        uint32_t* dk = last ? keys_out : ((p % 2 == 0) ? keys_tmp : const_cast<uint32_t*>(keys_in));
-        uint32_t* dv = last ? vals_out : ((p % 2 == 0) ? vals_tmp : const_cast<uint32_t*>(vals_in));
-        const int shift = p * db;
-        k_radix_upsweep<<<ntiles, kThreads, 0, s>>>(src_k, d_count, shift, mask, tile_hist, ntiles);
-        k_radix_scan<<<mask + 1, 1024, 0, s>>>(tile_hist, ntiles, row_total);
-        k_radix_downsweep<<<ntiles, kThreads, 0, s>>>(src_k, src_v, dk, dv, d_count, shift, mask, tile_hist,
-                                                      ntiles, row_total);
-        src_k = dk;
-        src_v = dv;
-    }
-    return cudaGetLastError();
+    return radix_passes(keys_in, vals_in, keys_tmp, vals_tmp, keys_out, vals_out, d_count, cap_count, key_bits, 8, tile_hist,
+                        row_total, s, nullptr);
 }
 
 }  // namespace hr
