@@ -506,7 +506,7 @@ int enqueue_render(hr_batch* b) {
     cudaStream_t s = c->stream;
     int rc;
     if ((rc = cuda_check(c, cudaMemsetAsync(b->d_work.p, 0, sizeof(uint32_t), s), "batch work reset"))) return rc;
-    return launch_jobs(c, dev<Job>(b->d_jobs), dev<uint32_t>(b->d_tile_off), b->nsc, dev<uint32_t>(b->d_work),
+    return launch_jobs(c, dev<Job>(b->d_jobs), dev<uint32_t>(b->d_tile_off), b->nsc, b->ntiles, dev<uint32_t>(b->d_work),
                        b->tile_w, b->block_threads, b->persist_blocks, false, s);
 }
 

@@ -230,10 +230,10 @@ uint32_t job_tiles(const Job& j, int32_t tw);
 // resident blocks per SM of the job kernel for a block size (pt: the path-tracing variant)
 int job_blocks_per_sm(int32_t block_threads, bool pt);
 // launch the persistent job kernel over njobs jobs whose tile prefix sums are d_tile_off
-// (njobs + 1 entries); *d_work must be zero.  pt selects the variant for kJobPath jobs,
+// (njobs + 1 entries, the last of them ntiles); *d_work must be zero.  pt selects the variant for kJobPath jobs,
 // which runs only those; the other variant runs every other mode.
-int launch_jobs(hr_ctx* c, const Job* d_jobs, const uint32_t* d_tile_off, uint32_t njobs, uint32_t* d_work,
-                int32_t tile_w, int32_t block_threads, int32_t nblocks, bool pt, cudaStream_t s);
+int launch_jobs(hr_ctx* c, const Job* d_jobs, const uint32_t* d_tile_off, uint32_t njobs, uint32_t ntiles,
+                uint32_t* d_work, int32_t tile_w, int32_t block_threads, int32_t nblocks, bool pt, cudaStream_t s);
 
 // trace.cu
 int launch_trace_rays(hr_ctx* c, const float* org, const float* dir, uint32_t n, int32_t* id,

@@ -33,7 +33,7 @@ constexpr int kJobTT = 256;   // largest block of the persistent kernel
 #define HR_JOB_PT_SMEM_STATE 1   // path-tracing instance: path state in shared memory
 #endif
 #ifndef HR_JOB_PT_MIN_BLOCKS
-#define HR_JOB_PT_MIN_BLOCKS 4   // the same for the path-tracing instance (4: 64 registers)
+#define HR_JOB_PT_MIN_BLOCKS 3   // the same for the path-tracing instance (24 served requests: 7.43 ms, 64 registers 7.59)
 #endif
 
 // position of the q-th (0-based) set bit of m; m has more than q set bits
@@ -128,18 +128,20 @@ template <bool PT>
 __global__ __launch_bounds__(kJobTT, PT ? HR_JOB_PT_MIN_BLOCKS : HR_JOB_MIN_BLOCKS) void k_trace_jobs(const Job* __restrict__ jobs,
                                                                         const uint32_t* __restrict__ tile_off,
                                                                         uint32_t njobs, uint32_t* work,
-                                                                        int32_t tile_w,
+                                                                        int32_t tile_w, uint32_t width,
                                                                         unsigned long long* counter) {
     __shared__ TileCtx s_tile[kJobTT / 32];
     TileCtx& T = s_tile[threadIdx.x >> 5];
     const uint32_t lane = threadIdx.x & 31u;
-    const uint32_t ntiles = __ldg(tile_off + njobs);
+    // a warp takes `width` slots of a tile at a time: 32, or a part of it when the tiles would
+    // not fill the warps
+    const uint32_t split = 32u / width, nunits = __ldg(tile_off + njobs) * split;
     const uint32_t tw = (uint32_t)tile_w, th = 32u / tw;
     if (PT) {
         // path jobs: lanes regenerate paths (next sample of the pixel, or the next pixel of
         // the warp's tiles); a tile of another job is taken once the warp's paths are done
         constexpr uint32_t kNone = 0xffffffffu;
-        uint32_t cur_j = kNone, tile_local = 0, next = 32u, pend = kNone;
+        uint32_t cur_j = kNone, slot0 = 0, next = width, pend = kNone;
         bool more = true;
 #if HR_JOB_PT_SMEM_STATE
         // the path state lives in shared memory, so the traversal has the registers to itself
@@ -155,29 +157,29 @@ __global__ __launch_bounds__(kJobTT, PT ? HR_JOB_PT_MIN_BLOCKS : HR_JOB_MIN_BLOC
         PtCounts n;
         while (true) {
             while (more) {
-                if (next >= 32u) {
+                if (next >= width) {
                     if (pend == kNone) {
                         uint32_t t = 0;
                         if (lane == 0) t = atomicAdd(work, 1u);
                         t = __shfl_sync(kFullMask, t, 0);
-                        if (t >= ntiles) {
+                        if (t >= nunits) {
                             more = false;
                             break;
                         }
                         pend = t;
                     }
-                    const uint32_t j = find_segment(tile_off, njobs, pend);
+                    const uint32_t j = find_segment(tile_off, njobs, pend / split);
                     if (j != cur_j) {
                         if (__any_sync(kFullMask, ln.has)) break;   // finish this job's paths first
                         if (lane == 0) load_tile_ctx(T, jobs + j);
                         __syncwarp();
                         cur_j = j;
                     }
-                    tile_local = pend - __ldg(tile_off + j);
+                    slot0 = (pend - __ldg(tile_off + j) * split) * width;
                     pend = kNone;
                     next = 0;
                 }
-                if (path_refill(ln, T.cam, tile_local * 32u, &next, 32u, T.image_id, T.seed, T.fb) == 0u) break;
+                if (path_refill(ln, T.cam, slot0, &next, width, T.image_id, T.seed, T.fb) == 0u) break;
             }
             if (!__any_sync(kFullMask, ln.has)) break;   // the pool is dry and every path is done
             const bool cont = path_step<kTwoLevel, false, HR_JOB_PT_SEEK_STEPS>(T.s, T.g, T.pk, ln.p, ln.has, n);
@@ -189,10 +191,11 @@ __global__ __launch_bounds__(kJobTT, PT ? HR_JOB_PT_MIN_BLOCKS : HR_JOB_MIN_BLOC
     }
     uint32_t nrays = 0, nsrays = 0;
     while (true) {
-        uint32_t tile = 0;
-        if (lane == 0) tile = atomicAdd(work, 1u);
-        tile = __shfl_sync(kFullMask, tile, 0);
-        if (tile >= ntiles) break;
+        uint32_t unit = 0;
+        if (lane == 0) unit = atomicAdd(work, 1u);
+        unit = __shfl_sync(kFullMask, unit, 0);
+        if (unit >= nunits) break;
+        const uint32_t tile = unit / split, sl = (unit - tile * split) * width + lane;   // this lane's slot of the tile
         const uint32_t j = find_segment(tile_off, njobs, tile);
         if (lane == 0) load_tile_ctx(T, jobs + j);
         __syncwarp();
@@ -202,13 +205,13 @@ __global__ __launch_bounds__(kJobTT, PT ? HR_JOB_PT_MIN_BLOCKS : HR_JOB_MIN_BLOC
         bool valid;
         uint32_t pix;
         if (rays) {
-            pix = lt * 32u + lane;
-            valid = pix < (uint32_t)T.cam.w;
+            pix = lt * 32u + sl;
+            valid = lane < width && pix < (uint32_t)T.cam.w;
         } else {
             const uint32_t cw = (uint32_t)T.cam.w, chh = (uint32_t)T.cam.h;
             const uint32_t tx = (cw + tw - 1u) / tw;
-            const uint32_t x = (lt % tx) * tw + lane % tw, y = (lt / tx) * th + lane / tw;
-            valid = x < cw && y < chh;
+            const uint32_t x = (lt % tx) * tw + sl % tw, y = (lt / tx) * th + sl / tw;
+            valid = lane < width && x < cw && y < chh;
             pix = valid ? y * cw + x : 0u;
         }
         // Round 0 traces the list or camera rays (closest hit), the rounds after it the AO
@@ -340,14 +343,23 @@ int job_blocks_per_sm(int32_t block_threads, bool pt) {
     return nb > 0 ? nb : 1;
 }
 
-int launch_jobs(hr_ctx* c, const Job* d_jobs, const uint32_t* d_tile_off, uint32_t njobs, uint32_t* d_work,
-                int32_t tile_w, int32_t block_threads, int32_t nblocks, bool pt, cudaStream_t s) {
+int launch_jobs(hr_ctx* c, const Job* d_jobs, const uint32_t* d_tile_off, uint32_t njobs, uint32_t ntiles,
+                uint32_t* d_work, int32_t tile_w, int32_t block_threads, int32_t nblocks, bool pt, cudaStream_t s) {
     if (block_threads < 32 || block_threads > kJobTT || block_threads % 32 != 0)
         return set_error(c, HR_ERR_INVALID_ARG, "jobs: block of %d threads", block_threads);
     c->launches += 1;
     unsigned long long* ctr = c->counters.as<unsigned long long>();
-    if (pt) k_trace_jobs<true><<<nblocks, block_threads, 0, s>>>(d_jobs, d_tile_off, njobs, d_work, tile_w, ctr);
-    else k_trace_jobs<false><<<nblocks, block_threads, 0, s>>>(d_jobs, d_tile_off, njobs, d_work, tile_w, ctr);
+    // Slots of a tile that a warp takes at a time: 32, or a smaller power of two (at least 8)
+    // while the tiles do not fill the warps four times over, as a short launch is as long as
+    // its slowest warp.  24 requests over four scenes at 32 slots / filled once / twice / four
+    // times 10.3 / 9.8 / 7.8 / 7.7 ms, 16 over three 5.14 / 3.24 / 3.17 / 3.18; batches of 12 and 20
+    // small scenes 461 / 465 / 420 / 381 us and 574 / - / 574 / 490; 24 scenes of up to 150k
+    // triangles alike.
+    const uint64_t warps = (uint64_t)nblocks * (uint64_t)block_threads / 32u;
+    uint32_t width = 32u;
+    while (width > 8u && (uint64_t)ntiles * (32u / width) < 4u * warps) width /= 2u;
+    if (pt) k_trace_jobs<true><<<nblocks, block_threads, 0, s>>>(d_jobs, d_tile_off, njobs, d_work, tile_w, width, ctr);
+    else k_trace_jobs<false><<<nblocks, block_threads, 0, s>>>(d_jobs, d_tile_off, njobs, d_work, tile_w, width, ctr);
     return cuda_check(c, cudaGetLastError(), "jobs launch");
 }
 

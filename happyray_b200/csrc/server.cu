@@ -287,10 +287,10 @@ int launch_wave(hr_server* S, Wave& w, std::map<uint32_t, float>& times) {
         (rc = cuda_check(c, cudaMemsetAsync(dw, 0, 2 * sizeof(uint32_t), s), "work")))
         return rc;
     cudaEventRecord(S->wave_start[w.slot], s);
-    if (n_main && (rc = launch_jobs(c, dj, dt, n_main, dw, S->tile_w, S->block_threads, S->blocks_main, false, s)))
+    if (n_main && (rc = launch_jobs(c, dj, dt, n_main, ht[n_main], dw, S->tile_w, S->block_threads, S->blocks_main, false, s)))
         return rc;
-    if (n_pt && (rc = launch_jobs(c, dj + n_main, dt + tiles_pt0, n_pt, dw + 1, S->tile_w, S->block_threads,
-                                  S->blocks_pt, true, s)))
+    if (n_pt && (rc = launch_jobs(c, dj + n_main, dt + tiles_pt0, n_pt, ht[tiles_pt0 + n_pt], dw + 1, S->tile_w,
+                                  S->block_threads, S->blocks_pt, true, s)))
         return rc;
     cudaEventRecord(S->wave_trace_end[w.slot], s);
     for (auto& kv : times) {
