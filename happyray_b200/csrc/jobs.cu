@@ -350,14 +350,15 @@ int launch_jobs(hr_ctx* c, const Job* d_jobs, const uint32_t* d_tile_off, uint32
     c->launches += 1;
     unsigned long long* ctr = c->counters.as<unsigned long long>();
     // Slots of a tile that a warp takes at a time: 32, or a smaller power of two (at least 8)
-    // while the tiles do not fill the warps four times over, as a short launch is as long as
-    // its slowest warp.  24 requests over four scenes at 32 slots / filled once / twice / four
-    // times 10.3 / 9.8 / 7.8 / 7.7 ms, 16 over three 5.14 / 3.24 / 3.17 / 3.18; batches of 12 and 20
-    // small scenes 461 / 465 / 420 / 381 us and 574 / - / 574 / 490; 24 scenes of up to 150k
-    // triangles alike.
+    // while the tiles do not fill the warps four times over (path jobs) or 16 times (the
+    // others, whose tiles over dense cells trace all their AO samples one after another), as a
+    // launch is as long as its slowest warp.  24 requests over four scenes at 32 slots /
+    // filled once / twice / four times 10.3 / 9.8 / 7.8 / 7.7 ms, 16 over three 5.14 / 3.24 /
+    // 3.17 / 3.18.  Renders of 24 scenes of up to 150k triangles at 4 / 16 / 32 times 1.36 /
+    // 1.11 / 1.07 ms, their passes 1895 / 1650 / 1660 us; 20 small scenes 490 / 467 / 467.
     const uint64_t warps = (uint64_t)nblocks * (uint64_t)block_threads / 32u;
     uint32_t width = 32u;
-    while (width > 8u && (uint64_t)ntiles * (32u / width) < 4u * warps) width /= 2u;
+    while (width > 8u && (uint64_t)ntiles * (32u / width) < (pt ? 4u : 16u) * warps) width /= 2u;
     if (pt) k_trace_jobs<true><<<nblocks, block_threads, 0, s>>>(d_jobs, d_tile_off, njobs, d_work, tile_w, width, ctr);
     else k_trace_jobs<false><<<nblocks, block_threads, 0, s>>>(d_jobs, d_tile_off, njobs, d_work, tile_w, width, ctr);
     return cuda_check(c, cudaGetLastError(), "jobs launch");
