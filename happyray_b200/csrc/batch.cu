@@ -140,18 +140,20 @@ __global__ __launch_bounds__(kBT) void kb_count_pairs(const float4* __restrict__
     const DescRegs g = load_desc(descs + ch.x);
     const uint32_t t = ch.y + threadIdx.x;
     uint32_t n = 0;
+    __shared__ float4 s_tri[3 * kBT];   // the vertex records leave in whole lines (k_count_pairs)
     if (t < end) {
         f3 p[3], lo, hi;
         CRange r;
         tri_load(v, idx, t, p);
-        float4* q = tris + 3 * (size_t)t;
-        q[0] = make_float4(p[0].x, p[0].y, p[0].z, 0.0f);
-        q[1] = make_float4(p[1].x, p[1].y, p[1].z, 0.0f);
-        q[2] = make_float4(p[2].x, p[2].y, p[2].z, 0.0f);
+#pragma unroll
+        for (int k = 0; k < 3; ++k) s_tri[3 * threadIdx.x + k] = make_float4(p[k].x, p[k].y, p[k].z, 0.0f);
         tri_bbox(p, &lo, &hi);
         n = cell_range(lo, hi, g.bmin, g.rcp, g.res, &r);
         if (ranges_fit(g.res)) rng[t] = pack_range(r, n);
     }
+    __syncthreads();
+    const uint32_t nrec = 3u * min((uint32_t)kBT, end - ch.y);
+    for (uint32_t i = threadIdx.x; i < nrec; i += kBT) tris[3 * (size_t)ch.y + i] = s_tri[i];
     uint32_t tot;
     block_excl_scan<uint32_t, kBT>(n, &tot);
     if (threadIdx.x == 0) {

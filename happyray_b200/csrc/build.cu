@@ -110,18 +110,21 @@ __global__ __launch_bounds__(kBT) void k_count_pairs(const float4* __restrict__ 
         for (uint32_t c = blockIdx.x * kBT + threadIdx.x; c < g.ncells; c += gridDim.x * kBT) cell_count[c] = 0u;
     const uint32_t t = blockIdx.x * kBT + threadIdx.x;
     uint32_t n = 0;
+    // the vertex records leave through shared memory, so that a warp stores whole lines
+    __shared__ float4 s_tri[3 * kBT];
     if (t < ntri) {
         f3 p[3], lo, hi;
         CRange r;
         tri_load(v, idx, t, p);
-        float4* q = tris + 3 * (size_t)t;
-        q[0] = make_float4(p[0].x, p[0].y, p[0].z, 0.0f);
-        q[1] = make_float4(p[1].x, p[1].y, p[1].z, 0.0f);
-        q[2] = make_float4(p[2].x, p[2].y, p[2].z, 0.0f);
+#pragma unroll
+        for (int k = 0; k < 3; ++k) s_tri[3 * threadIdx.x + k] = make_float4(p[k].x, p[k].y, p[k].z, 0.0f);
         tri_bbox(p, &lo, &hi);
         n = cell_range(lo, hi, g.bmin, g.rcp, g.res, &r);
         if (rng && ranges_fit(g.res)) rng[t] = pack_range(r, n);
     }
+    __syncthreads();
+    const uint32_t t0 = blockIdx.x * kBT, nrec = 3u * min((uint32_t)kBT, ntri - t0);
+    for (uint32_t i = threadIdx.x; i < nrec; i += kBT) tris[3 * (size_t)t0 + i] = s_tri[i];
     uint32_t tot;
     block_excl_scan<uint32_t, kBT>(n, &tot);
     if (threadIdx.x == 0) block_sums[blockIdx.x] = tot;

@@ -373,7 +373,7 @@ __global__ __launch_bounds__(kBT, 3) void k_build_ug_small(SmallUG P) {
         PairRun run;
         if (n) run = {(uint32_t)r.lo[0] + (uint32_t)r.lo[1] * rx + (uint32_t)r.lo[2] * rxy,
                       (uint32_t)(r.hi[0] - r.lo[0]), (uint32_t)(r.hi[1] - r.lo[1]), rx, rxy, t};
-        block_write_runs<kBT, 2>(n, run, pre, P.keys_a, P.vals_a, cnt);
+        block_write_runs<kBT, 2, 896u>(n, run, pre, P.keys_a, P.vals_a, cnt);
     }
     if (!grid_barrier(P.bar, P.d)) return;
 

@@ -1,6 +1,7 @@
-"""Exact insertion of triangles over many cells (written by blocks instead of one thread)
-against the oracle, bit for bit: extents around the serial limit, the piece size and the
-per-axis tables, through the single launch and through the pipeline."""
+"""Insertion of triangles over many cells against the oracle, bit for bit, through the single
+launch and through the pipeline.  Exact: written by blocks instead of one thread; extents
+around the serial limit, the piece size and the per-axis tables.  By bounding box: blocks
+whose runs are staged in shared memory beside blocks with longer ones."""
 import numpy as np
 import pytest
 
@@ -22,20 +23,21 @@ def scene(cells_per_side, tilt, flat, seed):
     return v, np.arange(len(v), dtype=np.uint32).reshape(-1, 3)
 
 
+@pytest.mark.parametrize("exact", [True, False])
 @pytest.mark.parametrize("pipeline", [False, True])
 @pytest.mark.parametrize("side,tilt,flat,density", [(4, 0.0, 1.0, 1.0), (4, 1.0, 1.0, 5.0), (20, 0.0, 1.0, 5.0),
                                                     (45, 1.0, 1.0, 5.0), (130, 0.1, 0.01, 5.0), (330, 0.0, 1e-4, 130.0)])
-def test_large_triangles_exact(oracle, monkeypatch, pipeline, side, tilt, flat, density):
+def test_large_triangles(oracle, monkeypatch, exact, pipeline, side, tilt, flat, density):
     if pipeline:
         monkeypatch.setenv("HAPPYRAY_SMALL_BUILD_MAX_TRIS", "0")
     v, f = scene(side, tilt, flat, side)
     v4, bmin, bmax = oracle.lerp_bounds(v, v, 1.0)
-    b = oracle.build_ug(v4, f, bmin, bmax, density, True)
+    b = oracle.build_ug(v4, f, bmin, bmax, density, exact)
     with Engine(0) as e:
         e.upload(v, v, f, 1.0)
         e.set_uniform_density(density)
         for _ in range(3):   # the third replays the captured build
-            e.build(GRID_UNIFORM, True)
+            e.build(GRID_UNIFORM, exact)
             gi, cells, _, prims = e.grid_download()
             assert gi["res"] == tuple(b.grid.res) and gi["num_pairs"] == b.npairs
             assert np.array_equal(cells, b.cells) and np.array_equal(prims, b.prims)
