@@ -154,22 +154,18 @@ void expand_xyz(const float* xyz, float4* out, size_t n, int grid, cudaStream_t 
 namespace {
 
 
-constexpr uint32_t kPinnedRays = 32768;   // ray queries up to this size are staged (hr_trace_rays)
+// Ray queries whose rays and hits fit in this are put together in host memory (hr_trace_rays);
+// beyond it the copies in and out of the buffer cost more than the calls they save.
+constexpr size_t kStageMax = 256u << 10;
 
-// page-locked staging of at least `bytes`; false when there is none to be had
-bool ensure_pinned(hr_ctx* c, size_t bytes) {
-    if (c->pinned_bytes >= bytes) return true;
-    if (c->pinned) cudaFreeHost(c->pinned);
-    c->pinned = nullptr;
-    c->pinned_bytes = 0;
-    const size_t want = std::max<size_t>(bytes + bytes / 2, 1u << 16);
-    if (cudaMallocHost(&c->pinned, want) != cudaSuccess) {
-        cudaGetLastError();
-        c->pinned = nullptr;
-        return false;
-    }
-    c->pinned_bytes = want;
-    return true;
+// host staging of at least `bytes` (at most kStageMax); false when there is none to be had
+bool ensure_host_stage(hr_ctx* c, size_t bytes) {
+    if (c->host_stage_bytes >= bytes) return true;
+    const size_t want = bytes <= kStageMax / 4 ? kStageMax / 4 : kStageMax;
+    free(c->host_stage);
+    c->host_stage = malloc(want);
+    c->host_stage_bytes = c->host_stage ? want : 0;
+    return c->host_stage != nullptr;
 }
 
 // copy `frames` xyz frames from host to float4 device storage
@@ -272,7 +268,7 @@ void hr_destroy(hr_ctx* c) {
     cudaStreamSynchronize(c->stream);
     for (auto& e : c->ev) if (e) cudaEventDestroy(e);
     for (auto& e : c->rev) if (e) cudaEventDestroy(e);
-    if (c->pinned) cudaFreeHost(c->pinned);
+    free(c->host_stage);
     if (c->desc_pinned) cudaFreeHost(c->desc_pinned);
     if (c->own_stream) cudaStreamDestroy(c->stream);
     delete c;
@@ -568,11 +564,13 @@ hr_status hr_trace_rays(hr_ctx* c, const float* org, const float* dir, uint32_t 
         return launch_trace_rays(c, dorg, ddir, n, reinterpret_cast<int32_t*>(dout), reinterpret_cast<float*>(dout + b1),
                                  reinterpret_cast<float*>(dout + 2 * b1), reinterpret_cast<float*>(dout + 3 * b1), nullptr);
     };
-    // A small query goes through the context's page-locked buffer, one copy each way: the six
-    // copies of pageable arrays, each waited for by itself, cost more than tracing a few
-    // rays (64 rays 73 -> 38 us, 8000 135 -> 95, 32,000 205 -> 190).
-    if (n <= kPinnedRays && ensure_pinned(c, 2 * b3 + 4 * b1)) {
-        char* const h = static_cast<char*>(c->pinned);
+    // A small query goes through the context's host buffer, one copy each way: six copies of the
+    // caller's arrays, each waited for by itself, cost more than tracing a few rays (64 rays
+    // 98 -> 43 us, 1000 111 -> 59, 6000 118 -> 86; 10,000 through a larger buffer 129 -> 106,
+    // 32,000 184 -> 233).  The buffer is pageable: page-locked it gives 1 to 15 us more a call,
+    // but locking it takes 1 to 3 ms of a context's first query.
+    if (2 * b3 + 4 * b1 <= kStageMax && ensure_host_stage(c, 2 * b3 + 4 * b1)) {
+        char* const h = static_cast<char*>(c->host_stage);
         std::memcpy(h, org, b3);
         std::memcpy(h + b3, dir, b3);
         if ((rc = cuda_check(c, cudaMemcpyAsync(dev, h, 2 * b3, cudaMemcpyHostToDevice, c->stream), "ray upload")) ||

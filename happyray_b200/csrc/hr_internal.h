@@ -130,8 +130,8 @@ struct hr_ctx {
     hr::DevBuf hit_t, hit_tri, unocc, queue;          // AO wavefront: per-pixel hits, hit-pixel queue
     cudaEvent_t rev[8] = {};     // render kernel boundaries (timing mode)
     int nrender_ev = 0;
-    void* pinned = nullptr;      // pinned host staging
-    size_t pinned_bytes = 0;
+    void* host_stage = nullptr;  // host staging of small ray queries (pageable)
+    size_t host_stage_bytes = 0;
 };
 
 namespace hr {

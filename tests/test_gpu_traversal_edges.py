@@ -55,6 +55,16 @@ def test_ray_queries_around_round_and_warp_sizes(engine, oracle, kind, ntri, nra
     assert np.array_equal(occ.cpu().numpy().astype(bool), np.asarray(oracle.occluded(b, org, d, tmax)).astype(bool))
 
 
+def test_host_queries_around_the_staging_sizes(engine, oracle):
+    """Host arrays of 40 bytes a ray around 64 and 256 KiB, growing and shrinking."""
+    v, f = overlapping_triangles(300, 300)
+    b = build(engine, oracle, v, f, GRID_TWO_LEVEL)
+    for n in (1, 1638, 1639, 6553, 6554, 64, 6000):
+        org, d = rays(n, n)
+        for got, want in zip(engine.trace_rays(org, d), oracle.trace(b, org, d)):
+            assert np.array_equal(got, want)
+
+
 @pytest.mark.parametrize("kind", [GRID_UNIFORM, GRID_TWO_LEVEL])
 @pytest.mark.parametrize("res", [(1, 1), (7, 3), (33, 17), (130, 70)])
 def test_camera_rays_and_counters(engine, oracle, kind, res):
