@@ -19,7 +19,7 @@ def keys_of(kind, n, bits, rng):
 
 @pytest.mark.parametrize("kind", ["random", "equal", "runs"])
 @pytest.mark.parametrize("n,bits", [(1, 1), (31, 4), (2047, 5), (2048, 8), (2049, 9), (6145, 13), (70_001, 17),
-                                    (WIDE - 1, 23), (WIDE, 18), (WIDE + 4097, 32)])
+                                    (WIDE - 1, 23), (WIDE, 18), (WIDE + 4097, 32), (7_000_003, 24)])
 def test_radix_sort_edges(engine, kind, n, bits):
     import torch
     rng = np.random.default_rng(n + bits)
