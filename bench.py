@@ -1277,7 +1277,6 @@ def main():
         return
     peak, peak_kind = peaks()
     l2_peak = l2_read_gbs(stream)
-    tl = W["kind"] == 1   # two-level AO kernels refill lanes inside the traversal loop
     ao = ["k_ao_primary", "k_ao_samples", "k_ao_finish"]
     names = {0: ["k_render_primary"], 1: ["k_render_pt"], 3: ao}[W["mode"]]
     kbytes = {0: [b_primary + b_secondary], 1: [b_primary + b_secondary], 3: [b_primary, b_secondary, 0]}[W["mode"]]
