@@ -275,9 +275,12 @@ __global__ __launch_bounds__(kTT, HR_TRACE_MIN_BLOCKS) void k_ao_primary(Scene s
 // waits; once HR_AO_REFILL_MIN lanes wait (or no ray is left in flight) they take the next
 // (hit pixel, sample) items from the pool together, so a warp keeps most of its lanes
 // busy until the pool runs dry instead of waiting for its longest ray, and the divergent
-// ray set-up runs for many lanes at once.
+// ray set-up runs for many lanes at once.  A launch traces samples k0 .. k0 + spp - 1 of every
+// hit pixel: items are counted in 32 bits, so the host cuts the samples of a large image into
+// launches of at most kAoItems items (what the warps take past the end then fits too).
+constexpr uint32_t kAoItems = 1u << 31;
 template <int KIND, bool STATS>
-__global__ __launch_bounds__(kTT, HR_TRACE_MIN_BLOCKS) void k_ao_samples(Scene s, Cam cam, int32_t spp, float alpha_frac,
+__global__ __launch_bounds__(kTT, HR_TRACE_MIN_BLOCKS) void k_ao_samples(Scene s, Cam cam, uint32_t k0, uint32_t spp, float alpha_frac,
                                                               float alpha_abs, uint64_t seed, int32_t image_id,
                                                               const float* __restrict__ hit_t,
                                                               const uint32_t* __restrict__ hit_tri,
@@ -293,7 +296,7 @@ __global__ __launch_bounds__(kTT, HR_TRACE_MIN_BLOCKS) void k_ao_samples(Scene s
     }
     const float off = 0.01f * alpha;
     const f3 cpos = mk(cam.pos[0], cam.pos[1], cam.pos[2]);
-    const uint32_t nitems = *qcount * (uint32_t)spp;
+    const uint32_t nitems = *qcount * spp;
     const uint32_t lane = threadIdx.x & 31u, lt = (1u << lane) - 1u;
     // rays a warp holds at a time (as ray_width): fewer where the items would not fill the warps,
     // at least 8
@@ -318,7 +321,7 @@ __global__ __launch_bounds__(kTT, HR_TRACE_MIN_BLOCKS) void k_ao_samples(Scene s
             const uint32_t item = base + __popc(need & lt);
             if (((need >> lane) & 1u) && item < nitems) {
                 has = true;
-                const uint32_t qi = item / (uint32_t)spp, k = item % (uint32_t)spp;
+                const uint32_t qi = item / spp, k = k0 + item % spp;
                 pix = queue[qi];
                 const f3 d = primary_dir(cam, pix);
                 const float t = hit_t[pix];
@@ -628,8 +631,8 @@ int launch_render(hr_ctx* c, int32_t mode, int32_t image_id, float* d_fb) {
         // word 7: the hit-pixel queue length and the sample pool; word 8: the camera-ray pool
         uint32_t* qcount = reinterpret_cast<uint32_t*>(ctr + 7);
         if ((rc = cuda_check(c, cudaMemsetAsync(qcount, 0, 4 * sizeof(uint32_t), strm), "queue reset"))) return rc;
-        const int spp = c->ip.ao_samples;
-        c->launches += 3;
+        const uint32_t spp = (uint32_t)c->ip.ao_samples, part = std::max(1u, std::min(spp, kAoItems / n));
+        c->launches += 2;
         mark(0);
         // blocks of both kernels: all resident at once (the launch bounds allow HR_TRACE_MIN_BLOCKS per SM)
         const int nb = HR_TRACE_MIN_BLOCKS * c->num_sms;
@@ -640,13 +643,18 @@ int launch_render(hr_ctx* c, int32_t mode, int32_t image_id, float* d_fb) {
                 c->queue.as<uint32_t>(), qcount, ctr, qcount + 2, width);
         });
         mark(1);
-        by_kind(s.kind, st, [&](auto K, auto S) {
-            k_ao_samples<K(), S()><<<nb, kTT, 0, strm>>>(
-                s, k, spp, c->ip.ao_radius_frac, c->ip.ao_radius_abs, c->ip.seed, image_id, c->hit_t.as<float>(),
-                c->hit_tri.as<uint32_t>(), c->queue.as<uint32_t>(), qcount, c->unocc.as<uint32_t>(), ctr, qcount + 1);
-        });
+        for (uint32_t k0 = 0; k0 == 0 || k0 < spp; k0 += part) {
+            if (k0 && (rc = cuda_check(c, cudaMemsetAsync(qcount + 1, 0, sizeof(uint32_t), strm), "sample pool reset"))) return rc;
+            c->launches += 1;
+            by_kind(s.kind, st, [&](auto K, auto S) {
+                k_ao_samples<K(), S()><<<nb, kTT, 0, strm>>>(
+                    s, k, k0, std::min(part, spp - k0), c->ip.ao_radius_frac, c->ip.ao_radius_abs, c->ip.seed, image_id,
+                    c->hit_t.as<float>(), c->hit_tri.as<uint32_t>(), c->queue.as<uint32_t>(), qcount, c->unocc.as<uint32_t>(),
+                    ctr, qcount + 1);
+            });
+        }
         mark(2);
-        k_ao_finish<<<c->num_sms * 4, 256, 0, strm>>>(c->queue.as<uint32_t>(), qcount, c->unocc.as<uint32_t>(), spp,
+        k_ao_finish<<<c->num_sms * 4, 256, 0, strm>>>(c->queue.as<uint32_t>(), qcount, c->unocc.as<uint32_t>(), (int32_t)spp,
                                                       image_id, d_fb);
         mark(3);
         c->nrender_ev = 4;
