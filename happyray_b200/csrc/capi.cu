@@ -168,6 +168,26 @@ bool ensure_host_stage(hr_ctx* c, size_t bytes) {
     return c->host_stage != nullptr;
 }
 
+// Whether a query's arrays can be read and written by the host now, as its staging does:
+// ordinary memory, or page-locked memory once the stream is idle (work enqueued before the
+// call may still be filling the rays).  Device and managed memory is left to the copies.
+bool host_arrays(hr_ctx* c, const void* const* p, int n) {
+    bool locked = false;
+    for (int k = 0; k < n; ++k) {
+        cudaPointerAttributes a;
+        if (cudaPointerGetAttributes(&a, p[k]) != cudaSuccess) {
+            cudaGetLastError();
+            return false;
+        }
+        if (a.type != cudaMemoryTypeUnregistered && a.type != cudaMemoryTypeHost) return false;
+        locked = locked || a.type == cudaMemoryTypeHost;
+    }
+    if (!locked) return true;
+    const cudaError_t e = cudaStreamQuery(c->stream);
+    if (e != cudaSuccess) cudaGetLastError();
+    return e == cudaSuccess;
+}
+
 // copy `frames` xyz frames from host to float4 device storage
 int upload_frames(hr_ctx* c, const float* const* frames, uint32_t nframes, uint32_t nv, DevBuf& dst) {
     const size_t fbytes = (size_t)nv * 3 * sizeof(float);
@@ -569,7 +589,8 @@ hr_status hr_trace_rays(hr_ctx* c, const float* org, const float* dir, uint32_t 
     // 98 -> 43 us, 1000 111 -> 59, 6000 118 -> 86; 10,000 through a larger buffer 129 -> 106,
     // 32,000 184 -> 233).  The buffer is pageable: page-locked it gives 1 to 15 us more a call,
     // but locking it takes 1 to 3 ms of a context's first query.
-    if (2 * b3 + 4 * b1 <= kStageMax && ensure_host_stage(c, 2 * b3 + 4 * b1)) {
+    const void* const arrays[6] = {org, dir, id, t, u, v};
+    if (2 * b3 + 4 * b1 <= kStageMax && host_arrays(c, arrays, 6) && ensure_host_stage(c, 2 * b3 + 4 * b1)) {
         char* const h = static_cast<char*>(c->host_stage);
         std::memcpy(h, org, b3);
         std::memcpy(h + b3, dir, b3);
