@@ -67,24 +67,27 @@ __device__ __forceinline__ void store_hit(const Scene& s, uint32_t i, f3 o, f3 d
     if (STATS) { stats[2 * (size_t)i] = h.cells; stats[2 * (size_t)i + 1] = h.tests; }
 }
 
-template <int KIND, bool STATS>
+// the rays of a query: `width` a warp, or (POOL) from a pool
+struct RayShare {
+    RayPool pool;
+    uint32_t width;
+};
+template <class T, int HM, bool STATS, bool POOL, class Gen, class Fin>
+__device__ __forceinline__ void trace_query(const Scene& s, const G& g, const RayShare& w, Gen gen, Fin fin) {
+    if constexpr (POOL) trace_pool<T, HM, STATS>(s, g, w.pool, gen, fin);
+    else trace_shares<T, HM, STATS>(s, g, w.pool.n, w.width, gen, fin);
+}
+
+template <int KIND, bool STATS, bool POOL>
 __global__ __launch_bounds__(kTT, HR_TRACE_MIN_BLOCKS) void k_trace_rays(Scene s, const float* __restrict__ org, const float* __restrict__ dir,
-                                                    RayPool w, int32_t* __restrict__ oid, float* __restrict__ ot,
+                                                    RayShare w, int32_t* __restrict__ oid, float* __restrict__ ot,
                                                     float* __restrict__ ou, float* __restrict__ ov,
                                                     uint32_t* __restrict__ stats) {
     const G g = load_g(s.desc);
     gate_scene(s);
-    trace_pool<QueryTrav<KIND, STATS>, kHitClosest, STATS>(
-        s, g, w,
-        [&](uint32_t i, f3& o, f3& d, Hit&) {
-            load_ray(org, dir, i, o, d);
-            return true;
-        },
-        [&](uint32_t i, Hit& h, bool) {
-            f3 o, d;
-            load_ray(org, dir, i, o, d);
-            store_hit<STATS>(s, i, o, d, h, oid, ot, ou, ov, stats);
-        });
+    trace_query<QueryTrav<KIND, STATS>, kHitClosest, STATS, POOL>(
+        s, g, w, [&](uint32_t i, f3& o, f3& d, Hit&) { load_ray(org, dir, i, o, d); },
+        [&](uint32_t i, f3 o, f3 d, Hit& h) { store_hit<STATS>(s, i, o, d, h, oid, ot, ou, ov, stats); });
 }
 
 // Camera rays by pixel tile, `width` consecutive slots of the tile order per warp and
@@ -118,24 +121,18 @@ __global__ __launch_bounds__(kTT, HR_TRACE_MIN_BLOCKS) void k_trace_primary(Scen
 // the ray-file form of render mode 0 (SimpleRayTraverser::integrate,
 // SimpleRayTraverser.h:166-180): ray i traced (closest hit) and shaded by simpleShade into
 // pixel i, progressive blend
-template <int KIND>
+template <int KIND, bool POOL>
 __global__ __launch_bounds__(kTT, HR_TRACE_MIN_BLOCKS) void k_render_rays(Scene s, const float* __restrict__ org,
-                                                                     const float* __restrict__ dir, RayPool w,
+                                                                     const float* __restrict__ dir, RayShare w,
                                                                      int32_t image_id, float* __restrict__ fb,
                                                                      unsigned long long* counter) {
     const G g = load_g(s.desc);
     gate_scene(s);
     uint32_t nrays = 0;
-    trace_pool<QueryTrav<KIND, false>, kHitClosest, false>(
-        s, g, w,
-        [&](uint32_t i, f3& o, f3& d, Hit&) {
-            load_ray(org, dir, i, o, d);
-            return true;
-        },
-        [&](uint32_t i, Hit& h, bool) {
-            f3 o, d;
+    trace_query<QueryTrav<KIND, false>, kHitClosest, false, POOL>(
+        s, g, w, [&](uint32_t i, f3& o, f3& d, Hit&) { load_ray(org, dir, i, o, d); },
+        [&](uint32_t i, f3 o, f3 d, Hit& h) {
             float rgb[3];
-            load_ray(org, dir, i, o, d);
             simple_shade(s, h.hit, h.tri, o, d, rgb);
             for (int k = 0; k < 3; ++k) fb[3 * (size_t)i + k] = blend(fb[3 * (size_t)i + k], rgb[k], image_id);
             nrays += 1;
@@ -143,19 +140,18 @@ __global__ __launch_bounds__(kTT, HR_TRACE_MIN_BLOCKS) void k_render_rays(Scene 
     add_rays<false>(counter, false, nrays);
 }
 
-template <int KIND>
+template <int KIND, bool POOL>
 __global__ __launch_bounds__(kTT, HR_TRACE_MIN_BLOCKS) void k_occluded(Scene s, const float* __restrict__ org, const float* __restrict__ dir,
-                                                  const float* __restrict__ tmax, RayPool w, uint8_t* __restrict__ occ) {
+                                                  const float* __restrict__ tmax, RayShare w, uint8_t* __restrict__ occ) {
     const G g = load_g(s.desc);
     gate_scene(s);
-    trace_pool<QueryTrav<KIND, false>, kHitAny, false>(
+    trace_query<QueryTrav<KIND, false>, kHitAny, false, POOL>(
         s, g, w,
         [&](uint32_t i, f3& o, f3& d, Hit& h) {
             load_ray(org, dir, i, o, d);
             h.t = __ldg(tmax + i);
-            return true;
         },
-        [&](uint32_t i, Hit& h, bool) { occ[i] = h.hit ? 1 : 0; });
+        [&](uint32_t i, f3, f3, Hit& h) { occ[i] = h.hit ? 1 : 0; });
 }
 
 // mode 0: primary rays with barycentric false colour (SimpleIntegrator.h:41-126)
@@ -482,19 +478,29 @@ uint32_t camera_width(const hr_ctx* c, bool ao) {
     return ao ? ray_width(slots, warps, 4, 16) : ray_width(slots, warps / 4u, 1, 8);
 }
 
-// The pool of a ray query over n rays and its block count (blocks resident at once; the
-// launch bounds allow HR_TRACE_MIN_BLOCKS per SM).  A query that fits takes the fewest rays
+// Whether a launch on the context's stream may run beside another one of this context: a
+// launch that is being captured (its graph may be replayed on any stream) or one on the
+// per-thread stream.
+bool may_overlap(const hr_ctx* c) {
+    if (c->stream == cudaStreamPerThread) return true;
+    cudaStreamCaptureStatus st = cudaStreamCaptureStatusNone;
+    if (cudaStreamIsCapturing(c->stream, &st) != cudaSuccess) cudaGetLastError();
+    return st != cudaStreamCaptureStatusNone;
+}
+
+// How a query over n rays is shared out, and its block count (the launch bounds allow
+// HR_TRACE_MIN_BLOCKS blocks per SM at once).  A query that fits takes the fewest rays
 // per warp that still have all of them in flight at once (64 rays 0.044 -> 0.028 ms, 4096
-// rays in a 2M-triangle scene 0.130 -> 0.091); a larger one refills from the pool.
-void ray_pool(const hr_ctx* c, uint32_t n, uint32_t refill, RayPool* w, int* blocks) {
+// rays in a 2M-triangle scene 0.130 -> 0.091); a larger one refills from the pool, whose
+// words are the context's, unless the launch may overlap another one.
+RayShare ray_share(const hr_ctx* c, uint32_t n, uint32_t refill, bool* pool, int* blocks) {
     const uint64_t wpb = kTT / 32, warps = (uint64_t)c->num_sms * HR_TRACE_MIN_BLOCKS * wpb;
-    w->n = n;
-    w->width = 32u;
-    while (w->width > 1u && n <= warps * (w->width / 2u)) w->width /= 2u;
-    w->refill = std::min(refill, w->width);
-    const uint64_t want = ((uint64_t)n + w->width - 1) / w->width;   // warps
-    *blocks = (int)((std::min(want, warps) + wpb - 1) / wpb);
-    w->next = want > (uint64_t)*blocks * wpb ? c->counters.as<unsigned long long>() + 9 : nullptr;
+    RayShare w = {{n, refill, c->counters.as<unsigned long long>() + 9}, 32u};
+    while (w.width > 1u && n <= warps * (w.width / 2u)) w.width /= 2u;
+    const uint64_t want = ((uint64_t)n + w.width - 1) / w.width;   // warps
+    *pool = want > warps && !may_overlap(c);
+    *blocks = (int)((std::min(want, *pool ? warps : 2 * warps) + wpb - 1) / wpb);
+    return w;
 }
 
 int grid_for(const hr_ctx* c, uint32_t n) {
@@ -528,12 +534,13 @@ int launch_trace_rays(hr_ctx* c, const float* org, const float* dir, uint32_t n,
                       float* v, uint32_t* stats) {
     if (n == 0) return 0;
     Scene s = make_scene(c);
-    RayPool w;
+    bool pool;
     int nb;
-    ray_pool(c, n, kQueryRefill, &w, &nb);
+    const RayShare w = ray_share(c, n, kQueryRefill, &pool, &nb);
     c->launches += 1;
     by_kind(s.kind, stats != nullptr, [&](auto K, auto S) {
-        k_trace_rays<K(), S()><<<nb, kTT, 0, c->stream>>>(s, org, dir, w, id, t, u, v, stats);
+        if (pool) k_trace_rays<K(), S(), true><<<nb, kTT, 0, c->stream>>>(s, org, dir, w, id, t, u, v, stats);
+        else k_trace_rays<K(), S(), false><<<nb, kTT, 0, c->stream>>>(s, org, dir, w, id, t, u, v, stats);
     });
     return cuda_check(c, cudaGetLastError(), "trace_rays launch");
 }
@@ -554,26 +561,30 @@ int launch_trace_primary(hr_ctx* c, int32_t* id, float* t, float* u, float* v, u
 
 int launch_render_rays(hr_ctx* c, const float* org, const float* dir, uint32_t n, int32_t image_id, float* fb) {
     if (n == 0) return 0;
-    RayPool w;
+    bool pool;
     int nb;
-    ray_pool(c, n, kQueryRefill, &w, &nb);
+    const RayShare w = ray_share(c, n, kQueryRefill, &pool, &nb);
     c->launches += 1;
     const Scene s = make_scene(c);
     unsigned long long* ctr = c->counters.as<unsigned long long>();
     by_kind(s.kind, false, [&](auto K, auto) {
-        k_render_rays<K()><<<nb, kTT, 0, c->stream>>>(s, org, dir, w, image_id, fb, ctr);
+        if (pool) k_render_rays<K(), true><<<nb, kTT, 0, c->stream>>>(s, org, dir, w, image_id, fb, ctr);
+        else k_render_rays<K(), false><<<nb, kTT, 0, c->stream>>>(s, org, dir, w, image_id, fb, ctr);
     });
     return cuda_check(c, cudaGetLastError(), "render_rays launch");
 }
 
 int launch_occluded(hr_ctx* c, const float* org, const float* dir, const float* tmax, uint32_t n, uint8_t* occ) {
     if (n == 0) return 0;
-    RayPool w;
+    bool pool;
     int nb;
-    ray_pool(c, n, kShadowRefill, &w, &nb);
+    const RayShare w = ray_share(c, n, kShadowRefill, &pool, &nb);
     c->launches += 1;
     const Scene s = make_scene(c);
-    by_kind(s.kind, false, [&](auto K, auto) { k_occluded<K()><<<nb, kTT, 0, c->stream>>>(s, org, dir, tmax, w, occ); });
+    by_kind(s.kind, false, [&](auto K, auto) {
+        if (pool) k_occluded<K(), true><<<nb, kTT, 0, c->stream>>>(s, org, dir, tmax, w, occ);
+        else k_occluded<K(), false><<<nb, kTT, 0, c->stream>>>(s, org, dir, tmax, w, occ);
+    });
     return cuda_check(c, cudaGetLastError(), "occluded launch");
 }
 

@@ -589,55 +589,68 @@ __device__ __forceinline__ void hit_reset(Hit& h, float tmax) {
     h.t = tmax; h.u = 0.0f; h.v = 0.0f; h.tri = 0; h.hit = false; h.cells = 0; h.tests = 0;
 }
 
-// n rays shared out to the warps of a launch: at most `width` rays of a warp are in flight,
-// the first of them items warp * width ..., the others taken from the pool (next[0], which
-// counts from the first warps' items on; null when those are all) once `refill` of the
-// warp's lanes are idle.  next[0] and next[1] (warps that left) are zero between launches.
+// Traces n rays, `width` of them per warp at a time (grid stride): gen(item, o, d, h) sets up
+// ray `item` (h.t its limit), fin(item, o, d, h) takes its result.
+template <class T, int HM, bool STATS, class Gen, class Fin>
+__device__ __forceinline__ void trace_shares(const Scene& s, const G& g, uint32_t n, uint32_t width, Gen gen, Fin fin) {
+    const uint32_t lane = threadIdx.x & 31u, wpb = blockDim.x >> 5, units = n / width + (n % width != 0u ? 1u : 0u);
+    for (uint32_t unit = blockIdx.x * wpb + (threadIdx.x >> 5); unit < units; unit += gridDim.x * wpb) {
+        const uint32_t item = unit * width + lane;
+        const bool active = lane < min(width, n - unit * width);
+        Hit h;
+        hit_reset(h, FLT_MAX);
+        f3 o = mk(0.0f, 0.0f, 0.0f), d = mk(1.0f, 0.0f, 0.0f);
+        if (active) gen(item, o, d, h);
+        if (s.ntri != 0u) trace_lanes<T, HM, STATS>(s, g, o, d, HM == kHitAny, h, active);
+        if (active) fin(item, o, d, h);
+    }
+}
+
+// More rays than the launch has in flight: every warp starts with 32 and takes the others from
+// the pool once `refill` of its lanes are idle.  next[0] counts the rays handed out beyond the
+// first, next[1] the warps that left; both are zero between launches, which the last warp
+// sees to, so launches that share them must not overlap.
 struct RayPool {
-    uint32_t n, width, refill;
+    uint32_t n, refill;
     unsigned long long* next;
 };
 
-// Traces the rays of a pool: gen(item, o, d, h) sets up ray `item` (h.t its limit) and
-// returns whether there is one, fin(item, h, valid) takes its result.  A lane whose ray is
-// done waits until `refill` lanes of its warp (at most `width`) are; they then retire their
-// rays and take the next items together, so a warp keeps most of its lanes busy until the
-// pool is dry instead of stepping until its longest ray ends, and the set-up and the
-// result of a ray run for many lanes at once.
+// As trace_shares, from a pool.  A lane whose ray is done waits until `refill` lanes of its
+// warp are; they then retire their rays and take the next items together, so a warp keeps
+// most of its lanes busy until the pool is dry instead of stepping until its longest ray
+// ends, and the set-up and the result of a ray run for many lanes at once.
 template <class T, int HM, bool STATS, class Gen, class Fin>
 __device__ __forceinline__ void trace_pool(const Scene& s, const G& g, const RayPool& w, Gen gen, Fin fin) {
     const uint32_t lane = threadIdx.x & 31u, lt = (1u << lane) - 1u;
     const uint32_t wpb = blockDim.x >> 5, warps = gridDim.x * wpb;
-    const unsigned long long first = (unsigned long long)(blockIdx.x * wpb + (threadIdx.x >> 5)) * w.width;
     T q;
     q.st = 0;
     Hit h;
     hit_reset(h, FLT_MAX);
     f3 o = mk(0.0f, 0.0f, 0.0f), d = mk(1.0f, 0.0f, 0.0f);
     uint32_t item = 0;
-    bool has = false, valid = false, fresh = true, dry = false;
+    bool has = false, fresh = true, dry = false;
     while (true) {
         // lanes without a ray in flight: they retire theirs and take the next ones together
-        const uint32_t need = __ballot_sync(kFullMask, q.st == 0 && lane < w.width);
+        const uint32_t need = __ballot_sync(kFullMask, q.st == 0);
         if ((uint32_t)__popc(need) >= w.refill) {   // warp-uniform
-            if (has && q.st == 0) fin(item, h, valid);
+            if (has && q.st == 0) fin(item, o, d, h);
             if (q.st == 0) has = false;
             if (!dry) {
-                unsigned long long base = first;
+                unsigned long long base = (unsigned long long)(blockIdx.x * wpb + (threadIdx.x >> 5)) * 32u;
                 if (!fresh) {
-                    if (lane == 0)
-                        base = (unsigned long long)warps * w.width + atomicAdd(w.next, (unsigned long long)__popc(need));
+                    if (lane == 0) base = (unsigned long long)warps * 32u + atomicAdd(w.next, (unsigned long long)__popc(need));
                     base = __shfl_sync(kFullMask, base, 0);
                 }
                 fresh = false;
-                if (w.next == nullptr || base + (uint32_t)__popc(need) >= w.n) dry = true;
+                if (base + (uint32_t)__popc(need) >= w.n) dry = true;
                 const unsigned long long i = base + __popc(need & lt);
                 if (((need >> lane) & 1u) && i < w.n) {
                     item = (uint32_t)i;
                     has = true;
                     hit_reset(h, FLT_MAX);
-                    valid = gen(item, o, d, h);
-                    if (valid && s.ntri != 0u) q.start(s, g, o, d, h);
+                    gen(item, o, d, h);
+                    if (s.ntri != 0u) q.start(s, g, o, d, h);
                 }
             }
             if (!__any_sync(kFullMask, has)) break;   // the pool is dry and no ray is in flight
@@ -647,7 +660,7 @@ __device__ __forceinline__ void trace_pool(const Scene& s, const G& g, const Ray
         q.next(s, g, o, d, h, done);
     }
     // the last warp to leave clears the pool for the next launch
-    if (w.next && lane == 0 && atomicAdd(w.next + 1, 1ull) == warps - 1u) {
+    if (lane == 0 && atomicAdd(w.next + 1, 1ull) == warps - 1u) {
         w.next[0] = 0ull;
         w.next[1] = 0ull;
     }
