@@ -489,10 +489,30 @@ bool may_overlap(const hr_ctx* c) {
 }
 
 // How a query over n rays is shared out, and its block count (the launch bounds allow
-// HR_TRACE_MIN_BLOCKS blocks per SM at once).  A query that fits takes the fewest rays
-// per warp that still have all of them in flight at once (64 rays 0.044 -> 0.028 ms, 4096
-// rays in a 2M-triangle scene 0.130 -> 0.091); a larger one refills from the pool, whose
+// HR_TRACE_MIN_BLOCKS blocks per SM at once).  A query that fits takes the fewest rays per warp
+// that still have all of them in flight at once; a larger one refills from the pool, whose
 // words are the context's, unless the launch may overlap another one.
+//
+// A launch is as long as its slowest warp, and a warp with few rays is through sooner: its
+// lists are tested by all 32 lanes, its walks by the few.  So long lists cost no more work in
+// narrow warps, empty cells do.  Shadow rays from the surfaces of 6,366 clustered triangles,
+// 7,366 of them, at 1 / 2 / 4 / 8 / 32 a warp: 128 / 148 / 230 / 319 / 830 us.  Where cells
+// are mostly empty the time alone is shorter too, but beside other queries the work counts:
+// random rays in a 100k heightfield (first line) and rays from above into a uniform grid of
+// it, us a query alone / among three streams' / among eight's:
+//   rays     one ray per lane     this rule            32 a warp
+//   1024     121 / 40.1 / 15.6    76 / 26.6 / 10.8     118 / 40.1 / 15.6
+//            46 / 15.7 / 6.3      22 / 7.9 / 3.6       47 / 16.2 / 6.5
+//   8192     151 / 51.5 / 21.5    94 / 34.1 / 16.3     146 / 50.0 / 20.4
+//            52 / 18.1 / 7.9      33 / 13.4 / 12.3     53 / 18.8 / 8.0
+//   20,000   129 / 45.6 / 21.3    92 / 34.8 / 22.7     111 / 40.0 / 18.7
+//            57 / 20.2 / 9.3      41 / 15.8 / 12.6     52 / 18.4 / 8.2
+//   65,536   145 / 59.2 / 46.1    114 / 52.9 / 51.8    125 / 49.3 / 38.4
+//            61 / 24.9 / 22.0     49 / 28.0 / 27.5     55 / 23.1 / 20.0
+// Half of the warps for widths up to 4 and a third for 8 and 16 would lose nothing among eight
+// (8192: 36 / 12.9 / 6.0 in the second line), but took 1.5 times as long for the shadow rays
+// above, 652 us against 471 for 48,774 rays into crowded uniform cells, and rebuilds of 2M
+// triangles with 7,349 rays 404 us a pass against 382.
 RayShare ray_share(const hr_ctx* c, uint32_t n, uint32_t refill, bool* pool, int* blocks) {
     const uint64_t wpb = kTT / 32, warps = (uint64_t)c->num_sms * HR_TRACE_MIN_BLOCKS * wpb;
     RayShare w = {{n, refill, c->counters.as<unsigned long long>() + 9}, 32u};

@@ -72,3 +72,38 @@ def test_captured_queries_replayed_beside_others(hrlib, kind):
         assert torch.equal(occ, wocc) and torch.equal(fb, wfb)
     del graphs
     e.close()
+
+
+@pytest.mark.parametrize("kind", [GRID_UNIFORM, GRID_TWO_LEVEL])
+def test_ray_counts_around_every_share(hrlib, oracle, kind):
+    """Ray counts on both sides of each number of rays per warp (all warps with 1, 2, 4, 8
+    and 16 rays) and of the refilled pool, whose words the next query finds cleared."""
+    import torch
+    v, f = S.clusters(2000, seed=3)
+    e = Engine(0)
+    e.upload(v, v, f, 1.0)
+    e.set_uniform_density(5.0)
+    e.setGridDensities(0.0625, 2.0)
+    e.build(kind)
+    v4, bmin, bmax = oracle.lerp_bounds(v, v, 1.0)
+    b = (oracle.build_ug(v4, f, bmin, bmax, 5.0, True) if kind == GRID_UNIFORM
+         else oracle.build_tl(v4, f, bmin, bmax, 0.0625, 2.0))
+    full = in_flight()
+    warps = full // 32
+    org, d = scene_rays(v, 2 * full + 33, 9)
+    want = oracle.trace(b, org, d)
+    tmax = np.full(len(org), 0.3, np.float32)
+    occ_o = np.asarray(oracle.occluded(b, org, d, tmax)).astype(bool)
+    do, dd, dt = (torch.from_numpy(x).cuda() for x in (org, d, tmax))
+    sizes = [warps * w + k for w in (1, 2, 4, 8, 16) for k in (0, 1)]
+    sizes += [full, full + 1, 2 * full + 33, 7]
+    for n in sizes:
+        out, occ = hits(n), torch.full((n,), 7, dtype=torch.uint8, device="cuda")
+        torch.cuda.synchronize()
+        e.trace_rays_device(do, dd, n, *out)
+        e.occluded_device(do, dd, dt, n, occ)
+        e.sync()
+        for got, x in zip(out, want):
+            assert np.array_equal(got.cpu().numpy(), x[:n])
+        assert np.array_equal(occ.cpu().numpy().astype(bool), occ_o[:n])
+    e.close()
