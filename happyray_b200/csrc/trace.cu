@@ -501,10 +501,10 @@ bool may_overlap(const hr_ctx* c) {
 // random rays in a 100k heightfield (first line) and rays from above into a uniform grid of
 // it, us a query alone / among three streams' / among eight's:
 //   rays     one ray per lane     this rule            32 a warp
-//   1024     121 / 40.1 / 15.6    76 / 26.6 / 10.8     118 / 40.1 / 15.6
+//   1024     121 / 40.1 / 15.6    76 / 26.6 / 10.8     118 / 40.6 / 15.6
 //            46 / 15.7 / 6.3      22 / 7.9 / 3.6       47 / 16.2 / 6.5
-//   8192     151 / 51.5 / 21.5    94 / 34.1 / 16.3     146 / 50.0 / 20.4
-//            52 / 18.1 / 7.9      33 / 13.4 / 12.3     53 / 18.8 / 8.0
+//   8192     151 / 51.5 / 21.5    94 / 34.1 / 16.3     146 / 50.3 / 20.4
+//            52 / 18.1 / 7.9      33 / 13.4 / 12.3     54 / 18.8 / 8.0
 //   20,000   129 / 45.6 / 21.3    92 / 34.8 / 22.7     111 / 40.0 / 18.7
 //            57 / 20.2 / 9.3      41 / 15.8 / 12.6     52 / 18.4 / 8.2
 //   65,536   145 / 59.2 / 46.1    114 / 52.9 / 51.8    125 / 49.3 / 38.4
