@@ -343,7 +343,7 @@ static std::vector<uint8_t> build_graph_key(const hr_ctx* c, int32_t kind, int32
         k.insert(k.end(), b, b + n);
     };
     // the frame pair and weight are not part of it: the graph reads them from frame_sel
-    const int32_t ints[5] = {kind, exact, c->timing ? 1 : 0, c->num_sms, c->lerp_pending ? 1 : 0};
+    const int32_t ints[6] = {kind, exact, c->timing ? 1 : 0, c->num_sms, c->lerp_pending ? 1 : 0, B.sort_items};
     const uint32_t sizes[3] = {c->ntri, c->nverts, c->nkeyframes};
     const float dens_all[3] = {dens, c->leaf_density, c->ug_density};
     const size_t caps[4] = {B.cap_cells, B.cap_pairs, B.cap_leaf_pairs, B.cap_leaves};
@@ -478,7 +478,7 @@ static int build_once_impl(hr_ctx* c, int32_t kind, int32_t exact, uint32_t* ovf
             if ((rc = radix_sort_pairs(c, B.keys_a.as<uint32_t>(), B.vals_a.as<uint32_t>(), B.keys_b.as<uint32_t>(),
                                        B.vals_b.as<uint32_t>(), sorted_keys, B.prims.as<uint32_t>(), d_np, cap_pairs,
                                        key_bits, B.tile_hist.as<uint32_t>(), B.tile_hist.bytes,
-                                       B.row_total.as<uint32_t>(), s)))
+                                       B.row_total.as<uint32_t>(), s, B.sort_items)))
                 return rc;
             mark();
             if (!exact || nblocks == 0)   // k_write_big_pairs cleared them
@@ -516,7 +516,7 @@ static int build_once_impl(hr_ctx* c, int32_t kind, int32_t exact, uint32_t* ovf
             if ((rc = radix_sort_pairs(c, B.lkeys_a.as<uint32_t>(), B.lvals_a.as<uint32_t>(), B.lkeys_b.as<uint32_t>(),
                                        B.lvals_b.as<uint32_t>(), leaf_keys, B.prims.as<uint32_t>(), &d->npairs,
                                        B.cap_leaf_pairs, leaf_bits, B.tile_hist.as<uint32_t>(), B.tile_hist.bytes,
-                                       B.row_total.as<uint32_t>(), s)))
+                                       B.row_total.as<uint32_t>(), s, B.sort_items)))
                 return rc;
             mark();
             const int gleaves = std::max(1, std::min((int)((B.cap_leaves + 255) / 256), c->num_sms * 16));
@@ -660,6 +660,7 @@ static void fit_caps(hr_ctx* c, const GridDesc& hd, int32_t kind) {
         if (cap > want + want / 2) cap = want;   // only when the estimate is far above
     };
     fit(B.cap_pairs, B.seen_pairs);
+    B.sort_items = radix_items(c, hd.npairs, B.sort_items);
     if (kind == kTwoLevel) {
         B.seen_leaves = std::max(B.seen_leaves, (size_t)hd.nleaves);
         B.seen_leaf_pairs = std::max(B.seen_leaf_pairs, (size_t)hd.npairs);
@@ -673,6 +674,7 @@ int build_grid(hr_ctx* c, int32_t kind, int32_t exact) {
     if (c->built_kind != kind) {
         B.cap_pairs = 0; B.cap_leaf_pairs = 0; B.cap_leaves = 0;
         B.seen_pairs = B.seen_leaves = B.seen_leaf_pairs = 0;
+        B.sort_items = 0;
     }
     c->async_pending = false;
     for (int attempt = 0; attempt < 6; ++attempt) {
@@ -713,6 +715,8 @@ int build_async_result(hr_ctx* c, bool* fit) {
         *fit = false;
         c->built = false;
         grow_caps(c, c->host_desc, ovf);
+    } else {
+        c->g.sort_items = radix_items(c, c->host_desc.npairs, c->g.sort_items);
     }
     return 0;
 }

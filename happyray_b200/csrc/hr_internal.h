@@ -59,6 +59,7 @@ struct GridBuffers {
     // largest sizes seen by a completed build: the capacities (which size the count, scan
     // and sort launches) follow them with headroom instead of the first estimates
     size_t seen_pairs = 0, seen_leaves = 0, seen_leaf_pairs = 0;
+    int sort_items = 0;   // keys per thread that the last build's pairs call for (radix_items), 0: none built
 };
 
 struct Stats {
@@ -177,8 +178,11 @@ int build_small_uniform(hr_ctx* c, int32_t exact, int key_bits, bool* done);
 int radix_sort_pairs(hr_ctx* c, const uint32_t* keys_in, const uint32_t* vals_in,
                      uint32_t* keys_tmp, uint32_t* vals_tmp, uint32_t* keys_out, uint32_t* vals_out,
                      const uint32_t* d_count, size_t cap_count, int key_bits,
-                     uint32_t* tile_hist, size_t tile_hist_bytes, uint32_t* row_total, cudaStream_t s);
+                     uint32_t* tile_hist, size_t tile_hist_bytes, uint32_t* row_total, cudaStream_t s, int items = 0);
 size_t radix_tile_hist_words(size_t cap_count, int key_bits);
+// keys per thread of a sort of n keys; with `last`, the choice of an earlier sort, the same one
+// again unless n has left its side of the line by an eighth
+int radix_items(const hr_ctx* c, size_t n, int last = 0);
 // passes radix_sort_pairs makes for keys of key_bits bits (the output of an odd count ends in
 // the temporary buffers' pass parity: the caller picks keys_out accordingly)
 int radix_sort_passes(int key_bits);

@@ -429,7 +429,6 @@ static void radix_plan(int key_bits, int max_db, int* passes, int* db) {
     *db = (key_bits + *passes - 1) / *passes;
 }
 
-constexpr size_t kWideTileKeys = 148 * 4 * 2048;   // from this many keys on, tiles of 4096 keys
 constexpr int kMaxDigitBits = 9;   // context sorts; the allocation-free sort keeps 8 (its static scratch)
 
 int radix_sort_passes(int key_bits) {
@@ -438,9 +437,12 @@ int radix_sort_passes(int key_bits) {
     return passes;
 }
 
-// keys per thread of a sort over up to cap_count keys: tiles of 4096 keys halve the counts
-// and the per-tile work, but need more keys to fill the GPU (see k_radix_scatter)
-static int radix_items(size_t cap_count) { return cap_count >= kWideTileKeys ? 16 : 8; }
+// tiles of 4096 keys halve the counts and the per-tile work, but need more keys to fill the GPU:
+// four tiles of 2048 per SM (see k_radix_scatter)
+int radix_items(const hr_ctx* c, size_t n, int last) {
+    const size_t line = (size_t)c->num_sms * 4u * kTile;
+    return n >= (last == 16 ? line - line / 8u : line) ? 16 : 8;
+}
 
 size_t radix_tile_hist_words(size_t cap_count, int key_bits) {
     int passes, db;
@@ -467,7 +469,7 @@ static cudaError_t radix_pass(const uint32_t* sk, const uint32_t* sv, uint32_t* 
 // all passes of a plan with digits of at most max_db bits
 static cudaError_t radix_passes(const uint32_t* keys_in, const uint32_t* vals_in, uint32_t* keys_tmp, uint32_t* vals_tmp,
                                 uint32_t* keys_out, uint32_t* vals_out, const uint32_t* d_count, size_t cap_count,
-                                int key_bits, int max_db, uint32_t* tile_hist, uint32_t* row_total, cudaStream_t s,
+                                int key_bits, int max_db, int items, uint32_t* tile_hist, uint32_t* row_total, cudaStream_t s,
                                 uint64_t* launches) {
     int passes, db;
     radix_plan(key_bits, max_db, &passes, &db);
@@ -479,8 +481,8 @@ static cudaError_t radix_passes(const uint32_t* keys_in, const uint32_t* vals_in
         const bool last = p == passes - 1;
         uint32_t* dk = last ? keys_out : ((p % 2 == 0) ? keys_tmp : const_cast<uint32_t*>(keys_in));
         uint32_t* dv = last ? vals_out : ((p % 2 == 0) ? vals_tmp : const_cast<uint32_t*>(vals_in));
-        auto pass = db <= 8 ? (radix_items(cap_count) == 16 ? radix_pass<8, 16> : radix_pass<8, 8>)
-                            : (radix_items(cap_count) == 16 ? radix_pass<9, 16> : radix_pass<9, 8>);
+        auto pass = db <= 8 ? (items == 16 ? radix_pass<8, 16> : radix_pass<8, 8>)
+                            : (items == 16 ? radix_pass<9, 16> : radix_pass<9, 8>);
         const cudaError_t e = pass(sk, sv, dk, dv, d_count, cap_count, p * db, mask, tile_hist, row_total, s);
         if (e != cudaSuccess) return e;
         if (launches) *launches += 3;
@@ -493,23 +495,24 @@ static cudaError_t radix_passes(const uint32_t* keys_in, const uint32_t* vals_in
 int radix_sort_pairs(hr_ctx* c, const uint32_t* keys_in, const uint32_t* vals_in,
                      uint32_t* keys_tmp, uint32_t* vals_tmp, uint32_t* keys_out, uint32_t* vals_out,
                      const uint32_t* d_count, size_t cap_count, int key_bits,
-                     uint32_t* tile_hist, size_t tile_hist_bytes, uint32_t* row_total, cudaStream_t s) {
+                     uint32_t* tile_hist, size_t tile_hist_bytes, uint32_t* row_total, cudaStream_t s, int items) {
     // the histogram holds 2^digit words per tile: fewer key bits can need more of them
     if (radix_tile_hist_words(cap_count, key_bits) * sizeof(uint32_t) > tile_hist_bytes)
         return set_error(c, 4, "radix sort: histogram of %zu bytes is too small for %zu keys of %d bits",
                          tile_hist_bytes, cap_count, key_bits);
     return cuda_check(c, radix_passes(keys_in, vals_in, keys_tmp, vals_tmp, keys_out, vals_out, d_count, cap_count, key_bits,
-                                      kMaxDigitBits, tile_hist, row_total, s, &c->launches), "radix_sort_pairs");
+                                      kMaxDigitBits, items ? items : radix_items(c, cap_count), tile_hist, row_total, s,
+                                      &c->launches), "radix_sort_pairs");
 }
 
 // Same pass sequence as radix_sort_pairs, without a context (no status text, no launch
-// count); used by the allocation-free entry point.
+// count); used by the allocation-free entry point, whose 2^20 pairs at most take the smaller tiles.
 cudaError_t radix_sort_pairs_raw(const uint32_t* keys_in, const uint32_t* vals_in, uint32_t* keys_tmp,
                                  uint32_t* vals_tmp, uint32_t* keys_out, uint32_t* vals_out,
                                  const uint32_t* d_count, size_t cap_count, int key_bits, uint32_t* tile_hist,
                                  uint32_t* row_total, cudaStream_t s) {
-    return radix_passes(keys_in, vals_in, keys_tmp, vals_tmp, keys_out, vals_out, d_count, cap_count, key_bits, 8, tile_hist,
-                        row_total, s, nullptr);
+    return radix_passes(keys_in, vals_in, keys_tmp, vals_tmp, keys_out, vals_out, d_count, cap_count, key_bits, 8, 8,
+                        tile_hist, row_total, s, nullptr);
 }
 
 }  // namespace hr
