@@ -261,7 +261,7 @@ hr_status hr_create(hr_ctx** out, int32_t device, void* stream) {
     }
     for (auto& e : c->ev) cudaEventCreate(&e);
     for (auto& e : c->rev) cudaEventCreate(&e);
-    if (ensure(c, c->counters, 96)) { hr_destroy(c); return HR_ERR_OUT_OF_MEMORY; }   // 8 counter words, 4 pool words
+    if (ensure(c, c->counters, 96)) { hr_destroy(c); return HR_ERR_OUT_OF_MEMORY; }   // words: traverse.cuh
     cudaMemsetAsync(c->counters.p, 0, 96, c->stream);
     {   // default light: a 0.2 x 0.2 quad at z = 1 centred over (0.5, 0.5), emitting along -z
         const float corner[3] = {0.4f, 0.4f, 1.0f}, e1[3] = {0.2f, 0.0f, 0.0f}, e2[3] = {0.0f, 0.2f, 0.0f};
@@ -639,7 +639,7 @@ hr_status hr_occluded_device(hr_ctx* c, const float* org, const float* dir, cons
 }
 
 // device counter words: [0] rays, [2] cells, [3] tests of the primary pass; [4] rays,
-// [5] cells, [6] tests of the secondary pass; [1] index check; [7] AO queue length
+// [5] cells, [6] tests of the secondary pass; [1] index check (all words: traverse.cuh)
 static int read_counters(hr_ctx* c, uint64_t w[8], int32_t reset) {
     int rc;
     if ((rc = cuda_check(c, cudaMemcpyAsync(w, c->counters.p, 64, cudaMemcpyDeviceToHost, c->stream), "counters")))

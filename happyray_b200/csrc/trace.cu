@@ -113,7 +113,7 @@ __global__ __launch_bounds__(kTT, HR_TRACE_MIN_BLOCKS) void k_trace_primary(Scen
         const bool valid = slot != kNoSlot && tile_pixel(cam, slot, &i);
         Hit h;
         const f3 d = valid ? primary_dir(cam, i) : mk(1.0f, 0.0f, 0.0f);
-        trace_one<KIND, false, STATS>(s, g, o, d, FLT_MAX, h, valid);
+        trace_one<KIND, STATS>(s, g, o, d, FLT_MAX, h, valid);
         if (valid) store_hit<STATS>(s, i, o, d, h, oid, ot, ou, ov, stats);
     });
 }
@@ -166,7 +166,7 @@ __global__ __launch_bounds__(kTT, HR_TRACE_MIN_BLOCKS) void k_render_primary(Sce
         const bool valid = slot != kNoSlot && tile_pixel(cam, slot, &i);
         const f3 d = valid ? primary_sample_dir(cam, i, image_id, seed) : mk(1.0f, 0.0f, 0.0f);
         Hit h;
-        trace_one<KIND, false, STATS>(s, g, o, d, FLT_MAX, h, valid);
+        trace_one<KIND, STATS>(s, g, o, d, FLT_MAX, h, valid);
         if (valid) {
             float rgb[3];
             simple_shade(s, h.hit, h.tri, o, d, rgb);

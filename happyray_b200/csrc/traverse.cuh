@@ -1,5 +1,5 @@
-// traverse.cuh -- device-side grid traversal shared by the per-scene kernels (trace.cu) and
-// the batched persistent kernel (batch.cu).
+// traverse.cuh -- device-side grid traversal shared by the per-scene kernels (trace.cu), the
+// persistent job kernel of batches and servers (jobs.cu) and the hierarchy's (hier.cu).
 //
 // Reference path (javorkk/happyray):
 //   uniform DDA            src/RT/Algorithm/UGridTraverser.h:44-177
@@ -218,9 +218,7 @@ __device__ __forceinline__ bool test_lists(const Scene& s, f3 o, f3 d, uint32_t 
     return answered;
 }
 
-__device__ __forceinline__ int min_dim(float a, float b, float c) { return a < b ? (a < c ? 0 : 2) : (b < c ? 1 : 2); }
-
-// One DDA step along the axis of the smallest t (min_dim).  `pos` is a linear index that
+// One DDA step along the axis of the smallest t (the last of equal ones).  `pos` is a linear index that
 // moves by the axis' signed stride st, `left` the steps that stay inside the grid per axis
 // (-1 once the step left it) and dt the axis' constant t increment, so a step is a handful
 // of predicated adds with no divergence between the axes.  (Against recomputing the cell
@@ -666,15 +664,14 @@ __device__ __forceinline__ void trace_pool(const Scene& s, const G& g, const Ray
     }
 }
 
-// Closest hit (ANY = false) or any hit within (1e-4, tmax) on a grid of kind KIND
-// (kUniform or kTwoLevel).  The kind is a template argument so that a kernel holds the
-// registers of one traversal only.  Warp-synchronous.
-template <int KIND, bool ANY, bool STATS>
+// Closest hit within (1e-4, tmax) on a grid of kind KIND (kUniform or kTwoLevel).  The kind
+// is a template argument so that a kernel holds the registers of one traversal only.
+// Warp-synchronous.
+template <int KIND, bool STATS>
 __device__ __forceinline__ void trace_one(const Scene& s, const G& g, f3 o, f3 d, float tmax, Hit& h, bool active) {
     hit_reset(h, tmax);
     if (s.ntri == 0) return;
-    constexpr int HM = ANY ? kHitAny : kHitClosest;
-    trace_lanes<Trav<KIND, STATS>, HM, STATS>(s, g, o, d, false, h, active);
+    trace_lanes<Trav<KIND, STATS>, kHitClosest, STATS>(s, g, o, d, false, h, active);
 }
 
 // As trace_one, with the hit mode chosen per lane: any hit where `any` is set, closest
@@ -815,7 +812,10 @@ __device__ __forceinline__ bool tile_pixel(const Cam& c, uint32_t slot, uint32_t
 // Device counters (uint64 words): [0] rays, [2] cells, [3] triangle tests of the primary
 // pass; [4] rays, [5] cells, [6] tests of the secondary pass (AO samples, shadow rays);
 // word 1 holds the index check of the last upload, word 7 the AO hit-pixel queue length
-// (or the path tracer's tile pool) and the AO sample pool, word 8 the AO camera-ray pool.
+// (or the path tracer's tile pool) and the AO sample pool, word 8 the AO camera-ray pool:
+// those the host clears before each launch.  Words 9 and 10 are the ray queries' pool, zero
+// between launches: cleared with the others when the context is created, then by the last
+// warp of each query that used them (trace_pool).  Word 11 is not used.
 template <bool STATS>
 __device__ __forceinline__ void add_rays(unsigned long long* counter, bool secondary, uint32_t rays, uint32_t cells = 0,
                                          uint32_t tests = 0) {
