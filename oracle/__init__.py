@@ -104,7 +104,7 @@ def lib():
                 "orc_hier_build": (C.c_int, [P, P, U32, P, U32, P, U32, F, F, P, C.POINTER(Grid), C.POINTER(P),
                                              C.POINTER(U32), C.POINTER(P), C.POINTER(U32), C.POINTER(P), C.POINTER(P),
                                              C.POINTER(U32)]),
-                "orc_hier_trace": (None, [C.POINTER(Hier), P, P, P, U32, C.c_int, P, P, P, P, P]),
+                "orc_hier_trace": (None, [C.POINTER(Hier), P, P, P, U32, C.c_int, P, P, P, P, P, P]),
             }
             for name, (res, args) in sig.items():
                 fn = getattr(L, name)
@@ -424,8 +424,10 @@ def hier_build(v, idx, obj_tri_counts, inst, top=1.2, leaf=1.2) -> BuiltHier:
                      _take(tc, 2 * g.ncells).reshape(-1, 2), _take(ii, ntp.value))
 
 
-def hier_trace(h: BuiltHier, org, dirs, tmax=None, anyhit=False):
-    """Closest hit (instance id, triangle id, t, u, v), or any hit below tmax."""
+def hier_trace(h: BuiltHier, org, dirs, tmax=None, anyhit=False, stats=False):
+    """Closest hit (instance id, triangle id, t, u, v), or any hit below tmax.  With stats also
+    an (n, 5) array: instance-grid cells, instance boxes tested, instances entered, object-grid
+    cells, triangle tests."""
     org = np.ascontiguousarray(org, np.float32)
     dirs = np.ascontiguousarray(dirs, np.float32)
     n = org.shape[0]
@@ -433,5 +435,6 @@ def hier_trace(h: BuiltHier, org, dirs, tmax=None, anyhit=False):
     out = [np.empty(n, np.int32), np.empty(n, np.int32), np.empty(n, np.float32), np.empty(n, np.float32),
            np.empty(n, np.float32)]
     s = h.struct()
-    lib().orc_hier_trace(C.byref(s), _p(org), _p(dirs), _p(tm), n, 1 if anyhit else 0, *[_p(a) for a in out])
-    return tuple(out)
+    work = np.empty((n, 5), np.uint32) if stats else None
+    lib().orc_hier_trace(C.byref(s), _p(org), _p(dirs), _p(tm), n, 1 if anyhit else 0, *[_p(a) for a in out], _p(work))
+    return tuple(out) + ((work,) if stats else ())

@@ -1328,7 +1328,9 @@ static inline void box_clip(const float *bmin, const float *bmax, f3 o, const fl
     *t1 = hmin(hmin(tf[0], tf[1]), tf[2]);
 }
 
-typedef struct { float t, u, v; int32_t inst, tri; } hhit;
+/* closest hit so far, and the work done for it: instance-grid cells, instance boxes tested,
+ * instances entered, object-grid cells, triangle tests */
+typedef struct { float t, u, v; int32_t inst, tri; uint32_t work[5]; } hhit;
 
 /* one instance: world box test, ray into object space, object grid DDA
  * (GeometryInstanceTraverser, TLGridHierarchyTraverser.h:45-205).  Returns 1 when the
@@ -1337,7 +1339,9 @@ static int hier_instance(const orc_hier *H, uint32_t ii, f3 o, f3 d, const float
     const orc_inst *I = &H->inst[ii];
     float te1, tx1;
     box_clip(I->bmin, I->bmax, o, rcp, &te1, &tx1);
+    h->work[1]++;
     if (!(tx1 > te1 && tx1 >= 0.0f && te1 < h->t)) return 0;
+    h->work[2]++;
     const float *m = I->m;
     /* transformRay (TwoLevelGridHierarchy.h:636-646): rows of the world -> object map;
      * the direction is carried, not re-derived from its reciprocal */
@@ -1369,6 +1373,8 @@ static int hier_instance(const orc_hier *H, uint32_t ii, f3 o, f3 d, const float
         if (cell[0] < g->res[0] && cell[0] > -1 && cell[1] < g->res[1] && cell[1] > -1 && cell[2] < g->res[2] &&
             cell[2] > -1) {
             size_t c = g->cell_off + (uint32_t)cell[0] + (uint32_t)cell[1] * rx + (uint32_t)cell[2] * rxy;
+            h->work[3]++;
+            h->work[4] += H->obj_cells[2 * c + 1] - H->obj_cells[2 * c];
             for (uint32_t it = H->obj_cells[2 * c]; it < H->obj_cells[2 * c + 1]; ++it) {
                 uint32_t tri = H->prims[it];
                 f3 v0 = vtx(H->v4, H->idx[3 * (size_t)tri]);
@@ -1425,6 +1431,7 @@ static void trace_hier(const orc_hier *H, f3 o, f3 d, int anyhit, hhit *h) {
         if (cell[0] < g->res[0] && cell[0] > -1 && cell[1] < g->res[1] && cell[1] > -1 && cell[2] < g->res[2] &&
             cell[2] > -1) {
             size_t c = (uint32_t)cell[0] + (uint32_t)cell[1] * rx + (uint32_t)cell[2] * rxy;
+            h->work[0]++;
             for (uint32_t it = H->top_cells[2 * c]; it < H->top_cells[2 * c + 1]; ++it)
                 if (hier_instance(H, H->inst_ids[it], o, d, rcp, h) && anyhit) return;
         }
@@ -1437,14 +1444,16 @@ static void trace_hier(const orc_hier *H, f3 o, f3 d, int anyhit, hhit *h) {
 }
 
 void orc_hier_trace(const orc_hier *H, const float *org, const float *dir, const float *tmax, uint32_t n,
-                    int anyhit, int32_t *inst_id, int32_t *tri_id, float *t, float *u, float *v) {
+                    int anyhit, int32_t *inst_id, int32_t *tri_id, float *t, float *u, float *v, uint32_t *stats) {
 #pragma omp parallel for schedule(dynamic, 64)
     for (long long ii = 0; ii < (long long)n; ++ii) {
         size_t i = (size_t)ii;
         hhit h;
         h.t = tmax ? tmax[i] : FLT_MAX; h.u = 0.0f; h.v = 0.0f; h.inst = -1; h.tri = -1;
+        memset(h.work, 0, sizeof(h.work));
         trace_hier(H, ld3(org + 3 * i), ld3(dir + 3 * i), anyhit, &h);
         inst_id[i] = h.inst; tri_id[i] = h.tri;
         t[i] = h.inst >= 0 ? h.t : FLT_MAX; u[i] = h.u; v[i] = h.v;
+        if (stats) memcpy(stats + 5 * i, h.work, sizeof(h.work));
     }
 }

@@ -176,9 +176,11 @@ int orc_hier_build(const float *v4, const uint32_t *idx, uint32_t ntri, const ui
                    orc_obj *objs, orc_grid *top, uint32_t **obj_cells, uint32_t *nobj_cells, uint32_t **prims,
                    uint32_t *npairs, uint32_t **top_cells, uint32_t **inst_ids, uint32_t *ntop_pairs);
 /* closest hit (tmax NULL: unbounded), or any hit below tmax[i] (anyhit = 1: inst_id >= 0
- * marks an occluded ray); inst_id / tri_id -1 on a miss */
+ * marks an occluded ray); inst_id / tri_id -1 on a miss.  stats (or NULL): 5 words per ray,
+ * instance-grid cells, instance boxes tested, instances entered, object-grid cells, triangle
+ * tests */
 void orc_hier_trace(const orc_hier *H, const float *org, const float *dir, const float *tmax, uint32_t n,
-                    int anyhit, int32_t *inst_id, int32_t *tri_id, float *t, float *u, float *v);
+                    int anyhit, int32_t *inst_id, int32_t *tri_id, float *t, float *u, float *v, uint32_t *stats);
 
 #ifdef __cplusplus
 }
